@@ -159,7 +159,7 @@ int lcu_op_linear(void *y, int stride_y, const void *x, int stride_x, const void
     const bool tc = batched && tc_on && n > 8 && gemm_tc_supported(in, w_dt == LCU_Q8_0);
     if (tc) gemm_tc_set_scratch(nullptr, 0, nullptr, 0, nullptr);
     for (int t0 = 0; t0 < n;) {
-        int nt = batched ? 64 : gemv_max_tokens(in);
+        int nt = tc ? GEMM_TC_MAX_TOKENS : (batched ? 64 : gemv_max_tokens(in));
         if (nt > n - t0) nt = n - t0;
         if (nt == 3 && !batched) nt = 2;
         GemvArgs a{};

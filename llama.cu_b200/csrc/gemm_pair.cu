@@ -1,0 +1,313 @@
+// `Linear` for rounds of many tokens (llama.cu/src/op/linear.rs:17-120) on pairs of SMs: tcgen05.mma.cta_group::2.
+//
+// Bound by the tensor pipe from a few hundred tokens on.  A CTA that computes a 128 x 256 tile alone writes 48 KB of operands
+// to its shared memory and reads as much for 512 cycles of MMA, which is more than shared memory carries; two CTAs that share
+// a 256 x 256 tile hold half of the weights' rows each and feed both tensor cores from them: 32 KB.  Hence:
+//   - D[256 tokens x NT weight rows]: CTA r of a pair owns tokens 128 r .. 128 r + 127 (lanes of its TMEM) and loads those
+//     rows of x and half of the tile's weight rows.  Tokens on lanes: a thread holds consecutive outputs of one token, so
+//     the 16-byte epilogues need no exchange through shared memory (gemm_tc.cu has weights on lanes);
+//   - persistent: one pair per two SMs, accumulators double-buffered in TMEM (2 x 256 columns), so the epilogue of a tile runs
+//     under the MMAs of the next; tiles in token-major order, so that neighbouring pairs read the same weights from L2;
+//   - warp 0 of both CTAs: TMA producer; warp 1 of the even CTA: MMA issuer; warps 2..9: epilogue, two per TMEM quadrant.
+// Measured (products alone, weights beyond L2): 28672 x 4096 with 997 tokens 356 -> 195 us (1.20 PFLOP/s), with 8000 tokens 2543 ->
+// 1356 us (1.39 PFLOP/s; cuBLAS 1267 us), 4096 x 14336 with 997 tokens 115 -> 104 us, against one CTA per 128 x 256 tile.
+// Barriers `full` and `tmem_empty` count in the even CTA; `empty` and `tmem_full` are signalled in both by tcgen05.commit.
+// Every mbarrier wait is bounded as in gemm_tc.cu: on expiry a status bit is set and the remaining work is skipped.
+#include <map>
+#include <mutex>
+
+#include "gemv.cuh"
+#include "tc.cuh"
+#include "tc_linear.cuh"
+
+namespace lcu {
+
+constexpr int TP_THREADS = 320;
+constexpr int TP_BM = 128;                       // tokens per CTA
+constexpr int TP_A_BYTES = TP_BM * TC_BK * 2;
+constexpr int TP_STAGES = 7;
+constexpr int TP_COLS = 256;                     // TMEM columns of one accumulator
+
+struct TpShared {
+    unsigned long long full[TP_STAGES], empty[TP_STAGES], tmem_full[2], tmem_empty[2];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+__device__ __forceinline__ uint32_t tp_in_leader(uint32_t saddr) {  // the same place in the shared memory of the pair's even CTA
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(saddr));
+    return r;
+}
+// issued by one lane of a converged warp (tc.cuh)
+__device__ __forceinline__ void tp_tma_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];\n}"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tp_mma4(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(LCU_TC_MMA4("2") ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tp_commit_both(uint32_t bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
+                 ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+__device__ __forceinline__ void tp_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// NT: weight rows of a tile (a multiple of 64; SwiGLU: NT / 2 gate rows, then their NT / 2 up rows)
+template <class T>
+__global__ void __launch_bounds__(TP_THREADS, 1) __cluster_dims__(2, 1, 1)
+gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, int NT,
+                 int n_mt, int n_tiles, uint32_t idesc, uint32_t *status) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *smem = smem_raw + ((1024u - (tc_smem(smem_raw) & 1023u)) & 1023u);
+    const int half = NT / 2;
+    const int stage_bytes = TP_A_BYTES + half * 128;
+    TpShared *sh = reinterpret_cast<TpShared *>(smem + (size_t)TP_STAGES * (TP_A_BYTES + TP_COLS / 2 * 128));
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    if (a.pdl_trigger == 0) grid_dep_launch();
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int nkb = a.in / TC_BK;
+    const bool swiglu = a.epilogue == EPI_SWIGLU;
+    const int step = swiglu ? half : NT;  // outputs of a tile
+
+    if (tid == 0) {
+        for (int i = 0; i < TP_STAGES; ++i) {
+            tc_mbar_init(tc_smem(&sh->full[i]), 1);
+            tc_mbar_init(tc_smem(&sh->empty[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            tc_mbar_init(tc_smem(&sh->tmem_full[i]), 1);
+            tc_mbar_init(tc_smem(&sh->tmem_empty[i]), 16);  // a lane of every epilogue warp of both CTAs
+        }
+        sh->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&sh->tmem_base)), "r"(2 * TP_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    tp_cluster_sync();  // the peer's barriers exist
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = sh->tmem_base;
+
+    if (warp == 0) {
+        // ---------------- TMA producer of this CTA's operands; their bytes count on the even CTA's barrier.  Places in the ring,
+        // phases and coordinates run along: one warp issues everything, and four integer divisions per stage cost more than
+        // the stage's MMAs
+        const uint32_t full0 = tc_smem(&sh->full[0]), full0_leader = tp_in_leader(full0), smem0 = tc_smem(smem);
+        const int w_off = rank == 0 ? 0 : (swiglu ? a.di : half);
+        auto weights = [&](int slot, int kx, int nt) {
+            if (rank == 0) tc_warp_expect_tx(full0 + 8 * slot, (uint32_t)(2 * stage_bytes));
+            tp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes + TP_A_BYTES), &map_w, kx, nt * step + w_off, full0_leader + 8 * slot);
+        };
+        auto acts = [&](int slot, int kx, int mt) {
+            tp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes), &map_x, kx, (2 * mt + rank) * TP_BM, full0_leader + 8 * slot);
+        };
+        // the weights do not depend on the previous kernel: the first ring of them (of this CTA's first tile) is requested ahead
+        // of the wait
+        const int early = nkb < TP_STAGES ? nkb : TP_STAGES;
+        int slot = 0;
+        uint32_t phase = 1;
+        bool primed = false, stop = false;
+        for (int tile = pair; tile < n_tiles && !stop; tile += n_pairs) {
+            const int nt = tile / n_mt, mt = tile - nt * n_mt;
+            int kb = 0;
+            if (!primed) {
+                for (int j = 0; j < early; ++j) weights(j, j * TC_BK, nt);
+                grid_dep_wait();
+                for (int j = 0; j < early; ++j) acts(j, j * TC_BK, mt);
+                kb = early;
+                slot = early == TP_STAGES ? 0 : early;
+                phase = early == TP_STAGES ? 0 : 1;
+                primed = true;
+            }
+            for (; kb < nkb; ++kb) {
+                if (!tc_warp_wait(tc_smem(&sh->empty[0]) + 8 * slot, phase, &sh->abort_flag)) {
+                    if (lane == 0) atomicOr(status, 4u);
+                    sh->abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                weights(slot, kb * TC_BK, nt);
+                acts(slot, kb * TC_BK, mt);
+                if (++slot == TP_STAGES) { slot = 0; phase ^= 1u; }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // ---------------- MMA issuer
+            const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]);
+            const uint64_t desc0 = tc_desc(tc_smem(smem));
+            int ti = 0, slot = 0;
+            bool stop = false;
+            uint32_t phase = 0;
+            for (int tile = pair; tile < n_tiles && !stop; tile += n_pairs, ++ti) {
+                const int ab = ti & 1;
+                if (!tc_warp_wait(tc_smem(&sh->tmem_empty[ab]), ((uint32_t)(ti >> 1) & 1u) ^ 1u, &sh->abort_flag)) {
+                    if (lane == 0) atomicOr(status, 4u);
+                    sh->abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d_tmem = tmem + (uint32_t)(ab * TP_COLS);
+                for (int kb = 0; kb < nkb; ++kb) {
+                    if (!tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag)) {
+                        if (lane == 0) atomicOr(status, 4u);
+                        sh->abort_flag = 1;
+                        stop = true;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4), db = da + (TP_A_BYTES >> 4);
+                    tp_mma4(d_tmem, da, db, idesc, kb > 0 ? 1u : 0u);
+                    tp_commit_both(empty0 + 8 * slot);
+                    if (++slot == TP_STAGES) { slot = 0; phase ^= 1u; }
+                }
+                tp_commit_both(tc_smem(&sh->tmem_full[ab]));
+            }
+        }
+    } else if (warp >= 2) {
+        // ---------------- epilogue: a thread has one token; the two warps of a quadrant take half of the columns each
+        const int q = warp & 3, h = (warp - 2) >> 2;
+        int ti = 0;
+        grid_dep_wait();  // residual rows and the round descriptor are earlier kernels'
+        for (int tile = pair; tile < n_tiles; tile += n_pairs, ++ti) {
+            const int mt = tile % n_mt, nt = tile / n_mt;
+            const int ab = ti & 1;
+            if (!tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag)) {
+                atomicOr(status, 4u);
+                sh->abort_flag = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int n = mt * 2 * TP_BM + rank * TP_BM + q * 32 + lane;
+            const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * TP_COLS);
+            if (swiglu) {
+                for (int c0 = h * (half / 2); c0 < (h + 1) * (half / 2); c0 += 16) {
+                    uint32_t g[16], u[16];
+                    tc_ld16(acc + (uint32_t)c0, g);
+                    tc_ld16(acc + (uint32_t)(half + c0), u);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    TcPre pre;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const int first = nt * step + c0 + 8 * k;
+                        if (n >= a.n_tok || first + 8 > a.di) continue;
+                        float v[8], w[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) { v[i] = __uint_as_float(g[8 * k + i]); w[i] = __uint_as_float(u[8 * k + i]); }
+                        tc_finish<T>(a, n, first, v, w, pre);
+                    }
+                }
+            } else {
+                for (int c0 = h * half; c0 < (h + 1) * half; c0 += 32) {
+                    const int first = nt * step + c0;
+                    TcPre pre[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (n < a.n_tok && first + 8 * k + 8 <= a.out) tc_prefetch<T>(a, n, first + 8 * k, pre[k]);
+                    uint32_t r[32];
+                    tc_ld16(acc + (uint32_t)c0, r);
+                    tc_ld16(acc + (uint32_t)(c0 + 16), r + 16);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (n >= a.n_tok || first + 8 * k + 8 > a.out) continue;
+                        float v[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[8 * k + i]);
+                        tc_finish<T>(a, n, first + 8 * k, v, v, pre[k]);
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
+        }
+    }
+    // ---------------- tail: both CTAs are done with each other's barriers and accumulators
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    tp_cluster_sync();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TP_COLS) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------ host side
+
+static size_t tp_smem_bytes() { return 1024 + (size_t)TP_STAGES * (TP_A_BYTES + TP_COLS / 2 * 128) + sizeof(TpShared); }
+
+// Weight rows of a tile: the time of a stage goes with the rows that both operands bring (0.29 us for 256 + 128, 0.43 us for
+// 256 + 256), so the fewest rows that the busiest pair loads.
+static int tp_tile(int n_mt, int rows, int pairs) {
+    int NT = 256, best = 1 << 30;
+    for (int nt = 256; nt >= 128; nt -= 64) {
+        const int tiles = n_mt * ((rows + nt - 1) / nt);
+        const int cost = (tiles + pairs - 1) / pairs * (2 * TP_BM + nt);
+        if (cost < best) { best = cost; NT = nt; }
+    }
+    return NT;
+}
+
+bool gemm_pair_takes(const GemvArgs &a) {
+    const int min = tuning().tc_pair_min;
+    if (min <= 0 || a.n_tok < min || a.tiles || a.push.n || !tc_vec(a)) return false;
+    if (min == 1) return true;
+    const int rows = a.epilogue == EPI_SWIGLU ? 2 * a.di : a.out, n_mt = (a.n_tok + 2 * TP_BM - 1) / (2 * TP_BM), pairs = sm_count() / 2;
+    const int NT = tp_tile(n_mt, rows, pairs);
+    return 2 * n_mt * ((rows + NT - 1) / NT) > pairs;
+}
+
+template <class T>
+static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, bool dry) {
+    static std::mutex mu;
+    static std::map<int, bool> done;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!done[dev]) {
+            LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes()));
+            done[dev] = true;
+        }
+    }
+    if (dry) return LCU_OK;
+    const int pairs = sm_count() / 2;
+    const int n_mt = (a.n_tok + 2 * TP_BM - 1) / (2 * TP_BM);
+    const int outs = a.epilogue == EPI_SWIGLU ? a.di : a.out, per = a.epilogue == EPI_SWIGLU ? 2 : 1;
+    const int NT = tp_tile(n_mt, outs * per, pairs);
+    const int n_nt = (outs * per + NT - 1) / NT;
+    CUtensorMap mw, mx;
+    int rc = tc_make_map(&mw, a.w, dt, (uint64_t)a.out, (uint64_t)a.in, (uint64_t)a.in, (uint32_t)NT / 2);
+    if (!rc) rc = tc_make_map(&mx, a.x, dt, (uint64_t)a.n_tok, (uint64_t)a.in, (uint64_t)a.stride_x, TP_BM);
+    if (rc) return rc;
+    const uint32_t fmt = dt == LCU_BF16 ? 1u : 0u;
+    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(2 * TP_BM >> 4) << 24);
+    const int tiles = n_mt * n_nt;
+    const int grid = 2 * (tiles < pairs ? tiles : pairs);
+    LCU_CHECK_CUDA(launch_kernel(gemm_pair_kernel<T>, dim3(grid), dim3(TP_THREADS), tp_smem_bytes(), s, pdl, a, mw, mx, NT, n_mt, tiles, idesc, status));
+    g_linear_last_ctas = grid;
+    return LCU_OK;
+}
+
+int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status) {
+    return dt == LCU_F16 ? tp_launch<__half>(a, dt, s, pdl, status, false) : tp_launch<__nv_bfloat16>(a, dt, s, pdl, status, false);
+}
+
+int gemm_pair_warm(int dt) {
+    GemvArgs a{};
+    return dt == LCU_F16 ? tp_launch<__half>(a, dt, nullptr, false, nullptr, true) : tp_launch<__nv_bfloat16>(a, dt, nullptr, false, nullptr, true);
+}
+
+}  // namespace lcu

@@ -36,6 +36,33 @@ __device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, vola
         if ((it & 255u) == 0 && (*abort_flag || tc_ns() - t0 > TC_WAIT_NS)) return false;
     }
 }
+// ---- forms for a whole converged warp: one elected lane issues, and nothing but the instruction depends on the lane, so the
+// compiler keeps operands and loop in uniform registers (issued from a `lane == 0` branch, four MMAs take 270 cycles to issue)
+__device__ __forceinline__ bool tc_warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    if (__all_sync(0xffffffffu, tc_mbar_try(bar, parity))) return true;
+    return __all_sync(0xffffffffu, tc_mbar_wait(bar, parity, abort_flag));
+}
+__device__ __forceinline__ void tc_warp_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n @e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(bar), "r"(bytes) : "memory");
+}
+// a K block of 64: four MMAs of K = 16 on operand tiles with 128-byte swizzle
+#define LCU_TC_MMA4(GROUP)                                                                                                          \
+    "{\n .reg .pred e, p, q;\n .reg .b64 a, b;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n setp.eq.b32 q, 0, 0;\n"       \
+    " @e tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], %1, %2, %3, p;\n add.u64 a, %1, 2;\n add.u64 b, %2, 2;\n"               \
+    " @e tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a, b, %3, q;\n add.u64 a, %1, 4;\n add.u64 b, %2, 4;\n"                 \
+    " @e tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a, b, %3, q;\n add.u64 a, %1, 6;\n add.u64 b, %2, 6;\n"                 \
+    " @e tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a, b, %3, q;\n}"
+__device__ __forceinline__ void tc_warp_mma4(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(LCU_TC_MMA4("1") ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc_warp_commit(uint32_t bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_warp_tma_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void tc_tma_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");

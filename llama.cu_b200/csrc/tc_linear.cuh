@@ -1,0 +1,155 @@
+// What the tcgen05 forms of the linear layer share: the vector epilogues and the operand maps.
+#pragma once
+#include "gemv.cuh"
+#include "tc.cuh"
+
+namespace lcu {
+
+constexpr int TC_BK = 64;  // K elements per stage (128 bytes: one swizzle row)
+
+#ifdef __CUDACC__
+// Vector form of the fused epilogues for one token and 8 consecutive outputs.  Everything a thread reads
+// from global memory for its items (residual, rotation table, page number) is fetched by tc_prefetch
+// before tc_finish stores anything: outputs may alias inputs (the residual is updated in place), so the
+// compiler cannot hoist those loads itself, and a chain of dependent round trips per item is what made
+// the scalar form slow.  Every access is 16 bytes.
+//   STORE / RESIDUAL / ROPE_KV: v[0..7] = 8 consecutive rows;  SWIGLU: v = gate, u = up of 8 pairs
+struct TcPre {
+    uint4 res;
+    float4 sn, cs;
+    uint32_t p;
+    int page;
+};
+
+template <class T>
+__device__ __forceinline__ void tc_prefetch(const GemvArgs &a, int n, int first, TcPre &pre) {
+    if (a.epilogue == EPI_RESIDUAL) {
+        pre.res = *reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(a.res) + (size_t)n * a.stride_res + first);
+    } else if (a.epilogue == EPI_ROPE_KV) {
+        const int sect = first < a.qd ? 0 : (first < a.qd + a.kvd ? 1 : 2);
+        const int rr = first - (sect == 0 ? 0 : (sect == 1 ? a.qd : a.qd + a.kvd));
+        const int e = rr % a.dh;
+        pre.p = a.pos[n];
+        if (sect < 2) {
+            const size_t ti = (size_t)pre.p * (a.dh >> 1) + (e >> 1);
+            pre.sn = *reinterpret_cast<const float4 *>(a.sin_t + ti);
+            pre.cs = *reinterpret_cast<const float4 *>(a.cos_t + ti);
+        }
+        if (sect > 0) pre.page = a.page_table[(size_t)a.tok_seq[n] * a.pt_stride + (pre.p >> a.geom.page_shift)];
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void tc_finish(const GemvArgs &a, int n, int first, float v[8], const float u[8], const TcPre &pre) {
+    T *dst = reinterpret_cast<T *>(a.y) + (size_t)n * a.stride_y + first;
+    if (a.epilogue == EPI_SWIGLU) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = swiglu_act(round_act<T>(v[i]), round_act<T>(u[i]));
+    } else if (a.epilogue == EPI_RESIDUAL) {
+        const uint32_t rw[4] = {pre.res.x, pre.res.y, pre.res.z, pre.res.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float2 rf = Act<T>::to_f2(rw[i]);
+            v[2 * i] += rf.x;
+            v[2 * i + 1] += rf.y;
+        }
+    } else if (a.epilogue == EPI_ROPE_KV) {
+        const int sect = first < a.qd ? 0 : (first < a.qd + a.kvd ? 1 : 2);
+        const int rr = first - (sect == 0 ? 0 : (sect == 1 ? a.qd : a.qd + a.kvd));
+        const int head = rr / a.dh, e = rr - head * a.dh;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = round_act<T>(v[i]);  // the projection is materialised before rope
+        if (sect < 2) {
+            const float sn[4] = {pre.sn.x, pre.sn.y, pre.sn.z, pre.sn.w}, cs[4] = {pre.cs.x, pre.cs.y, pre.cs.z, pre.cs.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float xa = v[2 * i], xb = v[2 * i + 1];
+                v[2 * i] = xa * cs[i] - xb * sn[i];
+                v[2 * i + 1] = xa * sn[i] + xb * cs[i];
+            }
+        }
+        if (sect > 0) {
+            const int slot = pre.p & (a.geom.page_tokens - 1);
+            dst = reinterpret_cast<T *>(a.kv_pool) + a.geom.block_off(pre.page, a.layer, sect - 1, head) + (size_t)slot * a.dh + e;
+        }
+    }
+    if (a.epilogue >= EPI_CAP)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = cap_logit(v[i], a.cap);
+    if (a.epilogue == EPI_STORE_F32 || a.epilogue == EPI_CAP_F32) {
+        float4 *f = reinterpret_cast<float4 *>(reinterpret_cast<float *>(a.y) + (size_t)n * a.stride_y + first);
+        f[0] = make_float4(v[0], v[1], v[2], v[3]);
+        f[1] = make_float4(v[4], v[5], v[6], v[7]);
+        return;
+    }
+    if (a.epilogue == EPI_XIELU) {
+        const float sp = softplus_f(__ldg(a.act_pq)), sq = softplus_f(__ldg(a.act_pq + 1));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = xielu_act(v[i], sp, sq);
+    }
+    if (a.epilogue == EPI_RELU2) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = relu2_act(v[i]);
+    }
+    if (a.epilogue == EPI_GLU) {
+        const float sc = a.row_scale ? a.row_scale[n] : 1.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = glu_act(sc * v[2 * i], sc * v[2 * i + 1], a.glu);
+        *reinterpret_cast<uint2 *>(reinterpret_cast<T *>(a.y) + (size_t)n * a.stride_y + first / 2) = make_uint2(Act<T>::pack(v[0], v[1]), Act<T>::pack(v[2], v[3]));
+        return;
+    }
+    uint4 o;
+    o.x = Act<T>::pack(v[0], v[1]); o.y = Act<T>::pack(v[2], v[3]); o.z = Act<T>::pack(v[4], v[5]); o.w = Act<T>::pack(v[6], v[7]);
+    if (a.push.n && (a.epilogue == EPI_STORE || a.epilogue == EPI_RESIDUAL)) {
+        // tensor parallelism: the partial goes to the owner's (scatter form) or every rank's all-reduce slot over peer memory
+        if (a.push.scatter_cols) {
+            *reinterpret_cast<uint4 *>(reinterpret_cast<T *>(a.push.slot[first / a.push.scatter_cols]) + (size_t)n * a.stride_y + first) = o;
+            return;
+        }
+        for (int k = 0; k < a.push.n; ++k)
+            *reinterpret_cast<uint4 *>(reinterpret_cast<T *>(a.push.slot[k]) + (size_t)n * a.stride_y + first) = o;
+        return;
+    }
+    *reinterpret_cast<uint4 *>(dst) = o;
+}
+#endif  // __CUDACC__
+
+// 2-D map of a row-major [rows, cols] matrix of 16-bit elements; box = 64 columns x box_rows rows, 128-byte swizzle
+inline int tc_make_map(CUtensorMap *m, const void *base, int dt, uint64_t rows, uint64_t cols, uint64_t row_stride,
+                       uint32_t box_rows) {
+    TcEncodeFn fn = tc_encode_fn();
+    if (!fn) {
+        set_error("gemm_tc: cuTensorMapEncodeTiled is not available");
+        return LCU_ERR_CUDA;
+    }
+    cuuint64_t gdim[2] = {cols, rows};
+    cuuint64_t gstr[1] = {row_stride * 2};
+    cuuint32_t box[2] = {TC_BK, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(m, dt == LCU_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                    const_cast<void *>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("gemm_tc: cuTensorMapEncodeTiled failed with %d (base %p, %llu x %llu, stride %llu)", (int)r, base,
+                  (unsigned long long)rows, (unsigned long long)cols, (unsigned long long)row_stride);
+        return LCU_ERR_CUDA;
+    }
+    return LCU_OK;
+}
+
+inline bool tc_vec(const GemvArgs &a) {  // whether the 16-byte epilogues apply
+    const bool f32 = a.epilogue == EPI_STORE_F32 || a.epilogue == EPI_CAP_F32;
+    bool ok = a.stride_y % (f32 ? 4 : 8) == 0 && ((uintptr_t)a.y % 16) == 0 && (a.epilogue == EPI_SWIGLU ? a.di % 8 == 0 : a.out % 8 == 0);
+    if (a.epilogue == EPI_RESIDUAL) ok = ok && a.stride_res % 8 == 0 && ((uintptr_t)a.res % 16) == 0;
+    if (a.epilogue == EPI_ROPE_KV)
+        ok = ok && a.dh % 8 == 0 && a.qd % 8 == 0 && a.kvd % 8 == 0 && ((uintptr_t)a.kv_pool % 16) == 0 && ((uintptr_t)a.sin_t % 16) == 0 &&
+             ((uintptr_t)a.cos_t % 16) == 0;
+    return ok;
+}
+
+// 256 x up to 256 tiles on pairs of SMs for rounds of many tokens (gemm_pair.cu); the arguments are those of gemm_tc_launch.
+bool gemm_pair_takes(const GemvArgs &a);
+int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status);
+int gemm_pair_warm(int dt);
+
+}  // namespace lcu
