@@ -5,10 +5,10 @@
 //
 // The GEMM is computed "swapped": D[128 weight rows x N tokens] += W_tile[128 x 64] · X[N x 64]^T,
 // so the weight dimension fills the 128-row MMA and the small token block is N (16, 32 or 64).
-//   - warp 0 (one lane): TMA producer — cp.async.bulk.tensor.2d loads of the weight tile (two
+//   - warp 0 (one elected lane): TMA producer — cp.async.bulk.tensor.2d loads of the weight tile (two
 //     64-row boxes) and of the activation tile into a ring of stages, 128-byte swizzle,
 //     completion on mbarriers.  Each weight byte is read once from HBM;
-//   - warp 1 (one lane): MMA issuer — four tcgen05.mma (K = 16 each) per stage, accumulating into
+//   - warp 1 (one elected lane): MMA issuer — four tcgen05.mma (K = 16 each) per stage, accumulating into
 //     TMEM; tcgen05.commit frees the stage and, after the last one, signals the epilogue;
 //   - warps 2..5: epilogue — tcgen05.ld of the 128 x N f32 accumulator into registers, staging
 //     through shared memory, then the same fused epilogues as the GEMV (gemv_epilogue: store,
@@ -57,7 +57,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
     float *stg = reinterpret_cast<float *>(smem + (size_t)n_stages * stage_bytes);  // [128][N + 1]
     TcShared *sh = reinterpret_cast<TcShared *>(reinterpret_cast<unsigned char *>(stg) + (size_t)TC_BM * (N + 1) * 4);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (a.pdl_trigger == 0) grid_dep_launch();
     const int nkb = a.in / TC_BK;  // K blocks of a whole row block
     const bool swiglu = a.epilogue == EPI_SWIGLU;
@@ -92,71 +92,81 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh->tmem_base;
 
-    if (warp == 0 && lane == 0) {
-        // ---------------- TMA producer: unit j of this CTA is (row block, K block) = divmod(u_begin + j, nkb)
+    if (warp == 0) {
+        // ---------------- TMA producer: units u_begin .. u_end - 1, unit = (row block, K block).  The whole warp runs the loop (one
+        // elected lane issues) and places, phases and coordinates run along: the divisions of a lane that works them out for
+        // every stage take longer than a stage's bytes (8B shape, f16, 32 sequences: 4.84 -> 4.28 ms per round; 33 tokens of the
+        // 1B shape 1.71 -> 1.51 ms, together with the peers' pieces of the cluster form requested at once)
         const int n_units = u_end - u_begin;
-        auto issue = [&](int j, bool weights, bool acts) {
-            const int u = u_begin + j, rb = u / nkb, kb = u - rb * nkb;
-            const int slot = j % n_stages;
-            const uint32_t bar = tc_smem(&sh->full[slot]);
-            const uint32_t dst = tc_smem(smem + (size_t)slot * stage_bytes);
-            const int kx = kb * TC_BK;
-            if (weights) {
-                tc_mbar_expect_tx(bar, (uint32_t)stage_bytes);
-                tc_tma_2d(dst, &map_w, kx, swiglu ? rb * 64 : rb * TC_BM, bar);
-                tc_tma_2d(dst + TC_A_BYTES / 2, &map_w, kx, swiglu ? a.di + rb * 64 : rb * TC_BM + 64, bar);
-            }
-            if (acts) tc_tma_2d(dst + TC_A_BYTES, &map_x, kx, 0, bar);
+        const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]), smem0 = tc_smem(smem);
+        const int row_step = swiglu ? 64 : TC_BM, second = swiglu ? a.di : 64;
+        auto weights = [&](int slot, int kb, int rb) {
+            const uint32_t bar = full0 + 8 * slot, dst = smem0 + (uint32_t)(slot * stage_bytes);
+            tc_warp_expect_tx(bar, (uint32_t)stage_bytes);
+            tc_warp_tma_2d(dst, &map_w, kb * TC_BK, rb * row_step, bar);
+            tc_warp_tma_2d(dst + TC_A_BYTES / 2, &map_w, kb * TC_BK, second + rb * row_step, bar);
+        };
+        auto acts = [&](int slot, int kb) {
+            tc_warp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes + TC_A_BYTES), &map_x, kb * TC_BK, 0, full0 + 8 * slot);
         };
         // The weights do not depend on the previous kernel: when this launch was allowed to start early
         // (programmatic dependent launch) the first ring of weight tiles is already streaming while the predecessor
         // finishes; the activation tiles of those stages follow once it has.
         const int first = n_units < n_stages ? n_units : n_stages;
-        for (int j = 0; j < first; ++j) issue(j, true, false);
+        int rb = u_begin / nkb, kb = u_begin - rb * nkb, kb_x = kb;
+        for (int j = 0; j < first; ++j) {
+            weights(j, kb, rb);
+            if (++kb == nkb) { kb = 0; ++rb; }
+        }
         grid_dep_wait();
-        for (int j = 0; j < first; ++j) issue(j, false, true);
-        for (int j = first; j < n_units && !sh->abort_flag; ++j) {
-            const int slot = j % n_stages;
-            const uint32_t parity = (uint32_t)(j / n_stages) & 1u;
-            if (!tc_mbar_wait(tc_smem(&sh->empty[slot]), parity ^ 1u, &sh->abort_flag)) {
-                atomicOr(status, 4u);
+        for (int j = 0; j < first; ++j) {
+            acts(j, kb_x);
+            if (++kb_x == nkb) kb_x = 0;
+        }
+        uint32_t phase = 0;
+        for (int j = first, slot = 0; j < n_units; ++j) {  // (only a full ring leaves units over)
+            if (!tc_warp_wait(empty0 + 8 * slot, phase, &sh->abort_flag)) {
+                if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
                 break;
             }
-            issue(j, true, true);
+            weights(slot, kb, rb);
+            acts(slot, kb);
+            if (++kb == nkb) { kb = 0; ++rb; }
+            if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer
-        int it = 0, ti = 0;
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (the whole warp, as above)
+        const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]);
+        const uint64_t desc0 = tc_desc(tc_smem(smem));
+        int slot = 0, ti = 0, kb0 = u_begin % nkb;
+        uint32_t phase = 0;
         for (int u = u_begin; u < u_end && !sh->abort_flag; ++ti) {
-            const int rb = u / nkb, kb0 = u - rb * nkb;
             const int kb1 = min(nkb, kb0 + (u_end - u));
-            u += kb1 - kb0;
             const int ab = ti & 1;
             // the epilogue must have drained this accumulator (two tiles ago)
-            if (!tc_mbar_wait(tc_smem(&sh->tmem_empty[ab]), ((uint32_t)(ti >> 1) & 1u) ^ 1u, &sh->abort_flag)) {
-                atomicOr(status, 4u);
+            if (!tc_warp_wait(tc_smem(&sh->tmem_empty[ab]), ((uint32_t)(ti >> 1) & 1u) ^ 1u, &sh->abort_flag)) {
+                if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t d_tmem = tmem + (uint32_t)(ab * acc_cols);
-            for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                const int slot = it % n_stages;
-                const uint32_t parity = (uint32_t)(it / n_stages) & 1u;
-                if (!tc_mbar_wait(tc_smem(&sh->full[slot]), parity, &sh->abort_flag)) {
-                    atomicOr(status, 4u);
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag)) {
+                    if (lane == 0) atomicOr(status, 4u);
                     sh->abort_flag = 1;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t sa = tc_smem(smem + (size_t)slot * stage_bytes), sb = sa + TC_A_BYTES;
-#pragma unroll
-                for (int k = 0; k < TC_BK / 16; ++k)
-                    tc_mma_f16(d_tmem, tc_desc(sa + k * 32), tc_desc(sb + k * 32), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-                tc_commit(tc_smem(&sh->empty[slot]));  // the stage is free once these MMAs have read it
+                const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4);
+                tc_warp_mma4(d_tmem, da, da + (TC_A_BYTES >> 4), idesc, kb > kb0 ? 1u : 0u);
+                tc_warp_commit(empty0 + 8 * slot);  // the stage is free once these MMAs have read it
+                if (++slot == n_stages) { slot = 0; phase ^= 1u; }
             }
-            tc_commit(tc_smem(&sh->tmem_full[ab]));     // accumulator complete
+            tc_warp_commit(tc_smem(&sh->tmem_full[ab]));     // accumulator complete
+            u += kb1 - kb0;
+            kb0 = 0;
         }
     } else if (warp >= 2) {
         // ---------------- epilogue warps: TMEM -> registers -> shared staging -> fused epilogue
@@ -382,7 +392,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
     float *stg = reinterpret_cast<float *>(smem + (size_t)n_stages * stage_bytes);  // [NS][TCK_LD]
     TcShared *sh = reinterpret_cast<TcShared *>(reinterpret_cast<unsigned char *>(stg) + (size_t)NS * TCK_LD * 4);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (a.pdl_trigger == 0) grid_dep_launch();
     const int nkb = a.in / TC_BK;
     const bool swiglu = a.epilogue == EPI_SWIGLU;
@@ -418,52 +428,52 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
     const uint32_t tmem = sh->tmem_base;
 
     bool ok = true;  // epilogue warps: the accumulator is complete
-    if (warp == 0 && lane == 0) {
-        // ---------------- TMA producer (weights of the first ring before the dependency wait, as in gemm_tc_kernel)
-        auto issue = [&](int j, bool weights, bool acts) {
-            const int slot = j % n_stages;
-            const uint32_t bar = tc_smem(&sh->full[slot]);
-            const uint32_t dst = tc_smem(smem + (size_t)slot * stage_bytes);
-            const int kx = (kb0 + j) * TC_BK;
-            if (weights) {
-                tc_mbar_expect_tx(bar, (uint32_t)stage_bytes);
-                tc_tma_2d(dst, &map_w, kx, wrow + (swiglu ? rb * 64 : rb * TC_BM), bar);
-                tc_tma_2d(dst + TC_A_BYTES / 2, &map_w, kx, wrow + (swiglu ? a.di + rb * 64 : rb * TC_BM + 64), bar);
-            }
-            if (acts) tc_tma_2d(dst + TC_A_BYTES, &map_x, kx, tb, bar);
+    if (warp == 0) {
+        // ---------------- TMA producer (weights of the first ring before the dependency wait, whole warp: as in gemm_tc_kernel)
+        const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]), smem0 = tc_smem(smem);
+        const int row_a = wrow + (swiglu ? rb * 64 : rb * TC_BM), row_b = swiglu ? wrow + a.di + rb * 64 : row_a + 64;
+        auto weights = [&](int slot, int kx) {
+            const uint32_t bar = full0 + 8 * slot, dst = smem0 + (uint32_t)(slot * stage_bytes);
+            tc_warp_expect_tx(bar, (uint32_t)stage_bytes);
+            tc_warp_tma_2d(dst, &map_w, kx, row_a, bar);
+            tc_warp_tma_2d(dst + TC_A_BYTES / 2, &map_w, kx, row_b, bar);
+        };
+        auto acts = [&](int slot, int kx) {
+            tc_warp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes + TC_A_BYTES), &map_x, kx, tb, full0 + 8 * slot);
         };
         const int first = n_units < n_stages ? n_units : n_stages;
-        for (int j = 0; j < first; ++j) issue(j, true, false);
+        for (int j = 0; j < first; ++j) weights(j, (kb0 + j) * TC_BK);
         grid_dep_wait();
-        for (int j = 0; j < first; ++j) issue(j, false, true);
-        for (int j = first; j < n_units && !sh->abort_flag; ++j) {
-            const int slot = j % n_stages;
-            const uint32_t parity = (uint32_t)(j / n_stages) & 1u;
-            if (!tc_mbar_wait(tc_smem(&sh->empty[slot]), parity ^ 1u, &sh->abort_flag)) {
-                atomicOr(status, 4u);
+        for (int j = 0; j < first; ++j) acts(j, (kb0 + j) * TC_BK);
+        uint32_t phase = 0;
+        for (int kb = kb0 + first, slot = 0; kb < kb1; ++kb) {
+            if (!tc_warp_wait(empty0 + 8 * slot, phase, &sh->abort_flag)) {
+                if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
                 break;
             }
-            issue(j, true, true);
+            weights(slot, kb * TC_BK);
+            acts(slot, kb * TC_BK);
+            if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issuer
-        for (int j = 0; j < n_units; ++j) {
-            const int slot = j % n_stages;
-            const uint32_t parity = (uint32_t)(j / n_stages) & 1u;
-            if (!tc_mbar_wait(tc_smem(&sh->full[slot]), parity, &sh->abort_flag)) {
-                atomicOr(status, 4u);
+        const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]);
+        const uint64_t desc0 = tc_desc(tc_smem(smem));
+        uint32_t phase = 0;
+        for (int j = 0, slot = 0; j < n_units; ++j) {
+            if (!tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag)) {
+                if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t sa = tc_smem(smem + (size_t)slot * stage_bytes), sb = sa + TC_A_BYTES;
-#pragma unroll
-            for (int k = 0; k < TC_BK / 16; ++k)
-                tc_mma_f16(tmem, tc_desc(sa + k * 32), tc_desc(sb + k * 32), idesc, (j > 0 || k > 0) ? 1u : 0u);
-            tc_commit(tc_smem(&sh->empty[slot]));
+            const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4);
+            tc_warp_mma4(tmem, da, da + (TC_A_BYTES >> 4), idesc, j > 0 ? 1u : 0u);
+            tc_warp_commit(empty0 + 8 * slot);
+            if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
-        tc_commit(tc_smem(&sh->tmem_full[0]));
+        tc_warp_commit(tc_smem(&sh->tmem_full[0]));
     } else if (warp >= 2) {
         ok = tc_mbar_wait(tc_smem(&sh->tmem_full[0]), 0u, &sh->abort_flag);
         if (!ok) {
@@ -512,16 +522,21 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
                 if (!(n < n_end && first + 8 <= (swiglu ? a.di : a.out))) continue;
                 float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, u[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 const uint32_t sv = tc_smem(stg + (size_t)nl * TCK_LD + 8 * c);
-                for (int p = 0; p < KS; ++p) {
-                    const float4 lo = tc_ld_dsmem4(sv, (uint32_t)p), hi = tc_ld_dsmem4(sv + 16, (uint32_t)p);
-                    v[0] += lo.x; v[1] += lo.y; v[2] += lo.z; v[3] += lo.w;
-                    v[4] += hi.x; v[5] += hi.y; v[6] += hi.z; v[7] += hi.w;
-                    if (swiglu) {
-                        const float4 l2 = tc_ld_dsmem4(sv + 64 * 4, (uint32_t)p), h2 = tc_ld_dsmem4(sv + 64 * 4 + 16, (uint32_t)p);
-                        u[0] += l2.x; u[1] += l2.y; u[2] += l2.z; u[3] += l2.w;
-                        u[4] += h2.x; u[5] += h2.y; u[6] += h2.z; u[7] += h2.w;
-                    }
-                }
+                // every peer's piece is requested before the first add (a round trip per peer otherwise); the sum runs in K order
+                auto sum = [&](uint32_t at, float o[8]) {
+                    float4 lo[8], hi[8];
+#pragma unroll
+                    for (int p = 0; p < 8; ++p)
+                        if (p < KS) { lo[p] = tc_ld_dsmem4(at, (uint32_t)p); hi[p] = tc_ld_dsmem4(at + 16, (uint32_t)p); }
+#pragma unroll
+                    for (int p = 0; p < 8; ++p)
+                        if (p < KS) {
+                            o[0] += lo[p].x; o[1] += lo[p].y; o[2] += lo[p].z; o[3] += lo[p].w;
+                            o[4] += hi[p].x; o[5] += hi[p].y; o[6] += hi[p].z; o[7] += hi[p].w;
+                        }
+                };
+                sum(sv, v);
+                if (swiglu) sum(sv + 64 * 4, u);
                 tc_finish<T>(a, n, first, v, u, pre[cnt]);
             }
         }
