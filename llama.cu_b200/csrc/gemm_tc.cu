@@ -575,6 +575,34 @@ static size_t tc_smem_bytes(int N, int stages) {
     return 1024 + (size_t)stages * (TC_A_BYTES + N * 128) + (size_t)TC_BM * (N + 1) * 4 + sizeof(TcShared) + 64;
 }
 
+// Clusters of ks CTAs of the cluster form that run at once on the current device (0: unknown, not possible).
+template <class T>
+static int tck_clusters(int ks, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::pair<int, std::pair<int, size_t>>, int> cache;
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    const auto key = std::make_pair(dev, std::make_pair(ks, smem));
+    const auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ks);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tck_kernel<T>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return cache[key] = n;
+}
+
 template <class T>
 static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool dry) {
     auto kernel = gemm_tc_kernel<T>;
@@ -622,28 +650,36 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
     if (rc) return rc;
     // ---- few row blocks: the CTAs of a row block form a cluster and merge through distributed shared memory
     {
-        // 1: where it measured faster than the stream-K split (64-token blocks: 6.23 -> 6.00 ms per 8B batch-64 step;
-        // very few row blocks: 11.2 -> 8.7 ms for one rank's share of the 70B shape; with 16..32 tokens and 32..48 row
-        // blocks the balanced stream-K split wins: 4.75 against 4.95 ms), 2: wherever it applies, 0: never
+        // tuning 1: where it costs less than the stream-K split, 2: wherever it applies, 0: never
         const int cluster_mode = tuning().tc_cluster;
         const int n_rb_c = (n_pairs + 63) / 64, nkb_c = a.in / TC_BK;
         const int n_tb = a.tiles ? a.n_tiles : (a.n_tok + N - 1) / N;  // token blocks: more than one for rounds of more than 256 tokens, and tiles
-        int KS = sms / (n_rb_c * n_tb);
-        if (KS > 8) KS = 8;
-        if (KS < 1) KS = 1;
-        while (KS > 1 && nkb_c / KS < 4) --KS;
-        // blocks of more than 64 tokens exist in this form only (clusters of one CTA where the matrix has row blocks to spare)
-        // 1: where it measured faster than the stream-K split: 64-token blocks, and matrices whose row blocks leave room
-        // for clusters of four and more (8B batch 32, per launch: O 20.9 -> 18.3 us, down 35.4 -> 32.9 us; the 48-row-block
-        // QKV matrix with clusters of three 26.8 -> 34.5 us, so it stays on stream-K)
+        const int stage_bytes = TC_A_BYTES + N * 128;
+        const int NS = N > 64 ? 64 : N;
+        const size_t fixed = 1024 + (size_t)NS * TCK_LD * 4 + sizeof(TcShared) + 64;
+        int st = (int)(((size_t)227 * 1024 - fixed) / stage_bytes);
+        if (st > TC_MAX_STAGES) st = TC_MAX_STAGES;
+        // CTAs per row block: a cluster lives in one GPC, so fewer of them fit than SMs / KS, and the ones left over start when the
+        // first wave is done (16 clusters of 8: 15 fit, 20 us instead of 8).  Cost in us, from CTAs' own clocks on the 1B and 8B
+        // shapes: start and merge of a wave 8, of a stream-K launch 13; a stage 0.25, but no less than the weights' bytes at 6 TB/s.
+        // Per round with 33 tokens of the 1B shape 1.51 -> 1.07 ms, 32 sequences of the 8B shape 4.28 -> 4.01 ms.
+        const int blocks = n_rb_c * n_tb;
+        const double bytes = 2e-6 * (double)a.out * a.in * n_tb / 6.;
+        auto cost = [&](double start, double stages) { return start + fmax(0.25 * stages, bytes); };
+        int KS = 1;
+        double best = 1e30;
+        for (int ks = 1; ks <= 8 && (ks == 1 || nkb_c / ks >= 4); ++ks) {
+            const int room = ks == 1 ? sms : blocks * ks <= sms ? tck_clusters<T>(ks, fixed + (size_t)st * stage_bytes) : 0;
+            if (room <= 0) continue;
+            const int waves = (blocks + room - 1) / room;
+            const double c = cost(8. * waves, (double)waves * ((nkb_c + ks - 1) / ks));
+            if (c < best) { best = c; KS = ks; }
+        }
         if (a.tiles) KS = 1;
-        const bool cluster_on = a.tiles || N > 64 || cluster_mode == 2 || (cluster_mode == 1 && (N == 64 || n_rb_c * 4 <= sms));
-        if (vec && cluster_on && (KS >= 2 || N > 64 || a.tiles)) {
-            const int stage_bytes = TC_A_BYTES + N * 128;
-            const int NS = N > 64 ? 64 : N;
-            const size_t fixed = 1024 + (size_t)NS * TCK_LD * 4 + sizeof(TcShared) + 64;
-            int st = (int)(((size_t)227 * 1024 - fixed) / stage_bytes);
-            if (st > TC_MAX_STAGES) st = TC_MAX_STAGES;
+        // blocks of more than 64 tokens, and tiles, exist in this form only (clusters of one CTA where the matrix has row blocks to spare)
+        const bool only = a.tiles || N > 64;
+        const bool cluster_on = only || (cluster_mode == 2 && KS >= 2) || (cluster_mode == 1 && best <= cost(13., (double)((blocks * nkb_c + sms - 1) / sms)));
+        if (vec && cluster_on) {
             const uint32_t idesc_c = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(n_rb_c * KS, n_tb);
