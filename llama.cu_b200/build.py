@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "liblcu.so")
-SOURCES = ["ctx.cu", "api.cu", "ops.cu", "gemv.cu", "attention.cu", "sample.cu", "comm.cu", "gemm_skinny.cu", "gemm_tc.cu", "gemm_pair.cu", "p2p.cu", "engine.cpp", "gguf.cpp",
+SOURCES = ["ctx.cu", "api.cu", "ops.cu", "gemv.cu", "attention.cu", "attention_tc.cu", "sample.cu", "comm.cu", "gemm_skinny.cu", "gemm_tc.cu", "gemm_pair.cu", "p2p.cu", "engine.cpp", "gguf.cpp",
            "stack.cu", "stack_pre.cu", "stack_ops.cu", "latent.cu", "latent_tc.cu", "gqa.cu", "delta.cu", "scan.cu", "moe.cu", "linear_f32.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

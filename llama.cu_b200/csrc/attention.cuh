@@ -36,6 +36,8 @@ struct AttnArgs {
     int pdl_trigger;
     float *part_o;        // [n_tok, nh, n_splits, dh]
     float *part_ml;       // [n_tok, nh, n_splits, 2]
+    int n_pages;          // tensor-core form: pages of the pool, and the status word of bounded waits
+    uint32_t *status;
     unsigned *counters;   // [n_tok, nkvh], zero before the first launch; the kernel re-zeroes them
 };
 
@@ -53,6 +55,11 @@ int attn_launch(const AttnArgs &a, int dt, cudaStream_t s, bool pdl, bool dry = 
 int attn_prefill_group_tokens(int nh, int nkvh);
 bool attn_prefill_supported(int pt_stride);
 int attn_prefill_launch(const AttnArgs &a, const void *groups_dev, int n_groups, int dt, cudaStream_t s, bool dry = false);
+
+// The same rounds on tcgen05 (attention_tc.cu): groups of up to attn_tc_group_tokens tokens, any number of pages.
+int attn_tc_group_tokens(int nh, int nkvh);
+bool attn_tc_takes(const KvGeom &g, int n_pages, const void *pool, unsigned longest);
+int attn_tc_launch(const AttnArgs &a, const void *groups_dev, int n_groups, int dt, cudaStream_t s, bool dry = false);
 
 // Appends k, v [seq, nkvh, dh] (strided) to linear caches at pos.. (the write half of
 // operators::attention_kv_cached as called from llama.cu/src/exec/step.rs:162-182).

@@ -42,6 +42,7 @@ struct Tuning {
     int tc = 1;                    // 0: keep the tcgen05 kernel out (mma.sync kernel for every batched round)
     int tc_block = 256;            // most tokens one tcgen05 launch takes (64, 128, 256): prefill rounds are cut into such blocks
     int tc_pair_min = 129;         // fewest tokens of a launch that takes 256-row tiles on pairs of SMs (0: none does)
+    int attn_tc = 1;               // attention of rounds that hold prompts on tcgen05: 0 never (mma.sync kernel), 1 where faster, 2 always
     int tc_cluster = 1;            // cluster split-K form of the tcgen05 kernel: 0 never, 1 where it measured faster, 2 wherever it applies
     int stack_pdl = 1;             // layered models, small rounds: every launch is a programmatic dependent of its predecessor
     int stack_fuse = 1;            // layered models, rounds of one or two decoded tokens: norms and residual as GEMV prologues (1: where it measured faster, 2: always)

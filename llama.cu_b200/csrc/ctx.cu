@@ -293,6 +293,7 @@ static int ctx_create(const lcu_model_desc &d, const lcu_layer_desc *layers, int
             a.n_tok = 1; a.nh = c->nh_l; a.nkvh = c->nkvh_l; a.dh = d.dh; a.n_splits = 1;
             rc = attn_launch(a, c->dt, nullptr, false, true);
             if (!rc) rc = attn_prefill_launch(a, nullptr, 0, c->dt, nullptr, true);
+            if (!rc) rc = attn_tc_launch(a, nullptr, 0, c->dt, nullptr, true);
         }
         if (rc) {
             lcu_ctx_destroy(c);
@@ -587,6 +588,7 @@ int lcu_set_tuning(lcu_ctx *c, const char *key, long long value) {
     else if (k == "tc") t.tc = value != 0;
     else if (k == "tc_block") { LCU_REQUIRE(value == 64 || value == 128 || value == 256, "set_tuning: tc_block = %lld (64, 128, 256)", value); t.tc_block = (int)value; }
     else if (k == "tc_pair_min") { LCU_REQUIRE(value >= 0, "set_tuning: tc_pair_min = %lld", value); t.tc_pair_min = (int)value; }
+    else if (k == "attn_tc") { LCU_REQUIRE(value >= 0 && value <= 2, "set_tuning: attn_tc = %lld (0..2)", value); t.attn_tc = (int)value; }
     else if (k == "tc_cluster") { LCU_REQUIRE(value >= 0 && value <= 2, "set_tuning: tc_cluster = %lld (0..2)", value); t.tc_cluster = (int)value; }
     else if (k == "stack_pdl") t.stack_pdl = value != 0;
     else if (k == "stack_fuse") { LCU_REQUIRE(value >= 0 && value <= 2, "set_tuning: stack_fuse = %lld (0..2)", value); t.stack_fuse = (int)value; }
@@ -826,8 +828,11 @@ int enqueue_round(lcu_ctx *c, const Round &r, lcu_kv_pair *out_dev, cudaStream_t
             const bool attn_pdl = pdl || (!batched && (pdl_edges & 1));
             a.early_kv = (attn_pdl && r.decode_only) ? 1 : 0;
             a.pdl_trigger = 1;
-            // rounds that hold prompts: 64 query rows per CTA share every K/V tile (prefill form)
-            if (r.n_groups > 0) rc = attn_prefill_launch(a, D + r.L.groups, r.n_groups, dt, s);
+            a.n_pages = c->n_pages;
+            a.status = c->dev_status;
+            // rounds that hold prompts: the rows of a group of tokens share every K/V tile
+            if (r.n_groups > 0 && r.attn_tc) rc = attn_tc_launch(a, D + r.L.groups, r.n_groups, dt, s);
+            else if (r.n_groups > 0) rc = attn_prefill_launch(a, D + r.L.groups, r.n_groups, dt, s);
             else rc = attn_launch(a, dt, s, attn_pdl);
             if (rc) return rc;
             ++launches;
@@ -1030,6 +1035,7 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
 
     // validate, then back every sequence with pages (KVCache::update, exec/group.rs:134-144)
     int n_tok = 0;
+    uint32_t longest = 0;  // context of a request after the round
     bool decode_only = true, any_sampling = false;
     for (int i = 0; i < n_req; ++i) {
         const lcu_req &q = reqs[i];
@@ -1041,6 +1047,7 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
             return LCU_ERR_OVERFLOW;
         }
         if (q.len != 1) decode_only = false;
+        if (q.pos + q.len > longest) longest = q.pos + q.len;
         n_tok += (int)q.len;
         if (args && !(args[i].temperature == 0.f || args[i].top_k == 1)) {
             LCU_REQUIRE(args[i].temperature > 0.f && args[i].top_p > 0.f && args[i].top_k >= 1, "step: bad sample args for request %d", i);
@@ -1123,9 +1130,10 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
             if (rc) return rc;
         }
         // prompts in the round: consecutive tokens of a request are grouped for the prefill form of attention
-        if (!c->stack && !decode_only && attn_prefill_supported(c->pt_stride)) {
+        r.attn_tc = !c->stack && !decode_only && attn_tc_takes(c->geom, c->n_pages, c->pool, longest);
+        if (!c->stack && !decode_only && (r.attn_tc || attn_prefill_supported(c->pt_stride))) {
             int32_t *hg = reinterpret_cast<int32_t *>(H + r.L.groups);
-            const int gt = attn_prefill_group_tokens(c->nh_l, c->nkvh_l);
+            const int gt = r.attn_tc ? attn_tc_group_tokens(c->nh_l, c->nkvh_l) : attn_prefill_group_tokens(c->nh_l, c->nkvh_l);
             int t0 = 0;
             for (int i = 0; i < n_req; ++i) {
                 for (uint32_t j = 0; j < reqs[i].len; j += gt) {

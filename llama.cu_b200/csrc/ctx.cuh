@@ -101,6 +101,7 @@ struct Round {
     int n_tok, n_req, n_fast;
     int n_out;     // rows of logits: one per request, or what lcu_step_logits asks for
     int n_groups;  // token groups for the prefill form of attention (0: decode form)
+    bool attn_tc = false;  // ... on tcgen05 (attention_tc.cu)
     bool any_sampling;
     bool decode_only;  // one new token per sequence
     float *logits_f32;  // lcu_step_logits: f32 logits of the asked rows go here, nothing is sampled
