@@ -12,9 +12,8 @@
 //     the commit behind S_t says that O_t is at rest as well;
 //   - warps 2..5 and 6..9: softmax of tile 0 and 1, one row per thread: maxima and sums need no exchange.  Weights are relative to the
 //     running maximum, as in attention.cu, so that they are rounded alike; O_t is rescaled in tensor memory where a row's moves.
-//     (A reference that moves by factors of 2^8 only takes 463 instead of 500 us for the 8000 tokens below, but rounds every
-//     weight in another place.)
-// Measured per layer: 8000 tokens of the 1B shape (dh 64) 1488 -> 500 us, 997 tokens of the 8B shape (dh 128) 85 -> 29 us, against
+//     (A reference that moves by factors of 2^8 only is no faster and rounds every weight in another place.)
+// Measured per layer: 8000 tokens of the 1B shape (dh 64) 1488 -> 456 us, 997 tokens of the 8B shape (dh 128) 85 -> 29 us, against
 // mma.sync on 64 rows per CTA.
 // Rows past the context are zeroed in the V tile (whatever a page holds there, its weight is zero).  Every wait is bounded: when one
 // runs out the CTA records a status bit, waits for its own copies, frees its tensor memory and returns.
