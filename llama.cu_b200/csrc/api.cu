@@ -156,7 +156,7 @@ int lcu_op_linear(void *y, int stride_y, const void *x, int stride_x, const void
     const bool batched = n > 4 && gemm_skinny_supported(in, w_dt == LCU_Q8_0) && out % 2 == 0;
     if (batched) gemm_skinny_set_scratch(nullptr, 0, nullptr, 0);  // the stand-alone operator owns no scratch: no K split
     const bool tc_on = tuning().tc != 0;
-    const bool tc = batched && tc_on && n > 8 && gemm_tc_supported(in, w_dt == LCU_Q8_0);
+    const bool tc = batched && tc_on && (n > 8 || w_dt == LCU_Q8_0) && gemm_tc_supported(in, w_dt == LCU_Q8_0);
     if (tc) gemm_tc_set_scratch(nullptr, 0, nullptr, 0, nullptr);
     for (int t0 = 0; t0 < n;) {
         int nt = tc ? GEMM_TC_MAX_TOKENS : (batched ? 64 : gemv_max_tokens(in));

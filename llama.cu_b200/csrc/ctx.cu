@@ -306,7 +306,8 @@ static int ctx_create(const lcu_model_desc &d, const lcu_layer_desc *layers, int
             if (!rc) rc = gemm_skinny_warm(c->qd, d.d, c->dt, q8);
             if (!rc) rc = gemm_skinny_warm(c->di_l, d.d, c->dt, q8);
             if (!rc) rc = gemm_skinny_warm(d.d, d.vocab & ~1, c->dt);
-            if (!rc && gemm_tc_supported(d.d, q8)) rc = gemm_tc_warm(c->dt);
+            if (!rc && gemm_tc_supported(d.d, false)) rc = gemm_tc_warm(c->dt);
+            if (!rc && q8) rc = gemm_tc_warm(c->dt, true);
             if (rc) {
                 lcu_ctx_destroy(c);
                 return rc;
@@ -742,7 +743,7 @@ int enqueue_round(lcu_ctx *c, const Round &r, lcu_kv_pair *out_dev, cudaStream_t
         if (batched && norm) {
             // launched as a programmatic dependent where the tcgen05 kernels follow (8B batch 32: 4.94 -> 4.85 ms, 70B per-rank
             // step: 8.35 -> 8.23 ms); ahead of the mma.sync kernels of Q8_0 rounds it costs (batch 16: 4.90 -> 5.34 ms)
-            const bool rms_pdl = tuning().rms_pdl && tc_on && n > 8 && gemm_tc_supported(proto.in, proto.w_q8);
+            const bool rms_pdl = tuning().rms_pdl && tc_on && (n > 8 || q8) && gemm_tc_supported(proto.in, proto.w_q8);
             int rc2 = op_rms_norm(c->hbuf, d.d, xin, stride_in, norm_w, norm_dt, d.eps, n, d.d, dt, s, pdl || rms_pdl);
             if (rc2) return rc2;
             ++launches;
@@ -754,7 +755,7 @@ int enqueue_round(lcu_ctx *c, const Round &r, lcu_kv_pair *out_dev, cudaStream_t
             // token blocks of 256 on the tcgen05 path (a weight tile is then streamed once per 256 tokens), all blocks in one
             // launch unless the output goes to peers or the tuning value asks for smaller launches; 64 otherwise
             const int tcb = tuning().tc_block < 256 || push ? tuning().tc_block : GEMM_TC_MAX_TOKENS;
-            const int blk = (tc_on && gemm_tc_supported(proto.in, proto.w_q8)) ? tcb : 64;
+            const int blk = (tc_on && gemm_tc_supported(proto.in, proto.w_q8) && !(proto.w_q8 && (push || n <= 128))) ? tcb : 64;
             if (batched) nt = n - t0 < blk ? n - t0 : blk;
             else {
                 nt = gemv_max_tokens(proto.in);
@@ -775,8 +776,8 @@ int enqueue_round(lcu_ctx *c, const Round &r, lcu_kv_pair *out_dev, cudaStream_t
             // launched early: the first weights are requested before waiting for the predecessor, then the activations
             a.early_prefetch = (pdl_in && early_prefetch == 1) ? 3 : early_prefetch;
             if (push) p2p_make_push(c->p2p, (size_t)t0 * stride_out * eb, &a.push, scatter_cols);
-            // more than 8 tokens: tcgen05 / TMEM kernel; 5..8: mma.sync kernel; up to 4: GEMV
-            const bool tc = batched && tc_on && nt > 8 && gemm_tc_supported(a.in, a.w_q8);
+            // more than 8 tokens, Q8_0 weights from 3 on: tcgen05 / TMEM kernel; up to 8: mma.sync kernel; 1 and 2: GEMV
+            const bool tc = batched && tc_on && (nt > 8 || a.w_q8) && gemm_tc_supported(a.in, a.w_q8);
             int rc2 = tc ? gemm_tc_launch(a, dt, s, pdl_in) : (batched ? gemm_skinny_launch(a, dt, s, pdl_in) : gemv_launch(a, dt, s, pdl_in));
             if (rc2) return rc2;
             ++launches;

@@ -26,10 +26,21 @@ constexpr int TP_THREADS = 320;
 constexpr int TP_BM = 128;                       // tokens per CTA
 constexpr int TP_A_BYTES = TP_BM * TC_BK * 2;
 constexpr int TP_STAGES = 7;
+// Q8_0 weights: tiles of 128 weight rows, 64 per CTA.  One more warp fetches their bytes and scales, 256 K elements at a time; eight
+// more turn them into pairs of f16 (tc_linear.cuh) and write them to shared memory as two operands, which the tensor pipe multiplies
+// one after the other.  Every 256 K elements have an accumulator of their own, and the epilogue warps add these up, rounded: the
+// tensor pipe cuts sums off, which thousands of products in a row show.  128 rows and not 256 because a thread then holds 64 sums.
+// Bound by shared memory: 88 KB per 64 K elements (x 16, bytes 8, pairs 16 written, x twice and pairs once read) are 690 cycles, the
+// MMAs 512; measured 830.  28672 x 4096 with 500 tokens in 170 us (0.69 PFLOP/s, counting each product once), eight passes of the
+// mma.sync kernel 1080 us; 500 tokens of the 8B shape 67.7 -> 16.5 ms.
+constexpr int TPQ_STAGES = 5, TPQ_GROUPS = 3;
+constexpr int TPQ_THREADS = TP_THREADS + 256 + 32;
+constexpr int TPQ_ROWS = 64;                              // weight rows of a CTA
+constexpr int TPQ_Q_BYTES = TPQ_ROWS * TQ_K, TPQ_G_BYTES = TPQ_Q_BYTES + TPQ_ROWS * (TQ_K / 32) * 2;
 constexpr int TP_COLS = 256;                     // TMEM columns of one accumulator
 
 struct TpShared {
-    unsigned long long full[TP_STAGES], empty[TP_STAGES], tmem_full[2], tmem_empty[2];
+    unsigned long long full[TP_STAGES], empty[TP_STAGES], tmem_full[2], tmem_empty[2], g_full[TPQ_GROUPS], g_empty[TPQ_GROUPS];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -57,16 +68,34 @@ __device__ __forceinline__ void tp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// waits for arrivals of both CTAs, and for what their threads wrote before them
+__device__ __forceinline__ bool tp_wait_both(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    auto attempt = [&]() {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        return __all_sync(0xffffffffu, ok != 0);
+    };
+    if (attempt()) return true;
+    const unsigned long long t0 = tc_ns();
+    for (unsigned it = 1;; ++it) {
+        if (attempt()) return true;
+        if ((it & 255u) == 0 && __any_sync(0xffffffffu, *abort_flag || tc_ns() - t0 > TC_WAIT_NS)) return false;
+    }
+}
+
 // NT: weight rows of a tile (a multiple of 64; SwiGLU: NT / 2 gate rows, then their NT / 2 up rows)
-template <class T>
-__global__ void __launch_bounds__(TP_THREADS, 1) __cluster_dims__(2, 1, 1)
-gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, int NT,
+template <class T, bool Q8>
+__global__ void __launch_bounds__(Q8 ? TPQ_THREADS : TP_THREADS, 1) __cluster_dims__(2, 1, 1)
+gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_x, int NT,
                  int n_mt, int n_tiles, uint32_t idesc, uint32_t *status) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (tc_smem(smem_raw) & 1023u)) & 1023u);
     const int half = NT / 2;
-    const int stage_bytes = TP_A_BYTES + half * 128;
-    TpShared *sh = reinterpret_cast<TpShared *>(smem + (size_t)TP_STAGES * (TP_A_BYTES + TP_COLS / 2 * 128));
+    constexpr int STAGES = Q8 ? TPQ_STAGES : TP_STAGES, COPIES = Q8 ? 2 : 1;
+    const int stage_bytes = TP_A_BYTES + COPIES * half * 128;
+    unsigned char *raw = smem + (size_t)STAGES * (TP_A_BYTES + (Q8 ? 2 * TPQ_ROWS : TP_COLS / 2) * 128);  // Q8_0: bytes and scales
+    TpShared *sh = reinterpret_cast<TpShared *>(raw + (Q8 ? TPQ_GROUPS * TPQ_G_BYTES : 0));
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (a.pdl_trigger == 0) grid_dep_launch();
@@ -76,13 +105,17 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
     const int step = swiglu ? half : NT;  // outputs of a tile
 
     if (tid == 0) {
-        for (int i = 0; i < TP_STAGES; ++i) {
-            tc_mbar_init(tc_smem(&sh->full[i]), 1);
+        for (int i = 0; i < STAGES; ++i) {
+            tc_mbar_init(tc_smem(&sh->full[i]), Q8 ? 5 : 1);  // Q8_0: and a lane of the two converting warps of both CTAs
             tc_mbar_init(tc_smem(&sh->empty[i]), 1);
         }
         for (int i = 0; i < 2; ++i) {
             tc_mbar_init(tc_smem(&sh->tmem_full[i]), 1);
             tc_mbar_init(tc_smem(&sh->tmem_empty[i]), 16);  // a lane of every epilogue warp of both CTAs
+        }
+        for (int i = 0; Q8 && i < TPQ_GROUPS; ++i) {
+            tc_mbar_init(tc_smem(&sh->g_full[i]), 1);
+            tc_mbar_init(tc_smem(&sh->g_empty[i]), 8);
         }
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -104,15 +137,15 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
         const uint32_t full0 = tc_smem(&sh->full[0]), full0_leader = tp_in_leader(full0), smem0 = tc_smem(smem);
         const int w_off = rank == 0 ? 0 : (swiglu ? a.di : half);
         auto weights = [&](int slot, int kx, int nt) {
-            if (rank == 0) tc_warp_expect_tx(full0 + 8 * slot, (uint32_t)(2 * stage_bytes));
-            tp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes + TP_A_BYTES), &map_w, kx, nt * step + w_off, full0_leader + 8 * slot);
+            if (rank == 0) tc_warp_expect_tx(full0 + 8 * slot, (uint32_t)(2 * (Q8 ? TP_A_BYTES : stage_bytes)));
+            if (!Q8) tp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes + TP_A_BYTES), &map_w, kx, nt * step + w_off, full0_leader + 8 * slot);
         };
         auto acts = [&](int slot, int kx, int mt) {
             tp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes), &map_x, kx, (2 * mt + rank) * TP_BM, full0_leader + 8 * slot);
         };
         // the weights do not depend on the previous kernel: the first ring of them (of this CTA's first tile) is requested ahead
         // of the wait
-        const int early = nkb < TP_STAGES ? nkb : TP_STAGES;
+        const int early = nkb < STAGES ? nkb : STAGES;
         int slot = 0;
         uint32_t phase = 1;
         bool primed = false, stop = false;
@@ -124,8 +157,8 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 grid_dep_wait();
                 for (int j = 0; j < early; ++j) acts(j, j * TC_BK, mt);
                 kb = early;
-                slot = early == TP_STAGES ? 0 : early;
-                phase = early == TP_STAGES ? 0 : 1;
+                slot = early == STAGES ? 0 : early;
+                phase = early == STAGES ? 0 : 1;
                 primed = true;
             }
             for (; kb < nkb; ++kb) {
@@ -137,7 +170,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 }
                 weights(slot, kb * TC_BK, nt);
                 acts(slot, kb * TC_BK, mt);
-                if (++slot == TP_STAGES) { slot = 0; phase ^= 1u; }
+                if (++slot == STAGES) { slot = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -145,10 +178,12 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
             // ---------------- MMA issuer
             const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]);
             const uint64_t desc0 = tc_desc(tc_smem(smem));
-            int ti = 0, slot = 0;
+            int ti = 0, slot = 0;  // accumulators taken: one per tile, Q8_0: per group of four K blocks
             bool stop = false;
             uint32_t phase = 0;
-            for (int tile = pair; tile < n_tiles && !stop; tile += n_pairs, ++ti) {
+            const int span = Q8 ? 4 : nkb;
+            const int n_acc = pair < n_tiles ? (n_tiles - pair + n_pairs - 1) / n_pairs * (nkb / span) : 0;
+            for (; ti < n_acc && !stop; ++ti) {
                 const int ab = ti & 1;
                 if (!tc_warp_wait(tc_smem(&sh->tmem_empty[ab]), ((uint32_t)(ti >> 1) & 1u) ^ 1u, &sh->abort_flag)) {
                     if (lane == 0) atomicOr(status, 4u);
@@ -158,8 +193,8 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d_tmem = tmem + (uint32_t)(ab * TP_COLS);
-                for (int kb = 0; kb < nkb; ++kb) {
-                    if (!tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag)) {
+                for (int kb = 0; kb < span; ++kb) {
+                    if (!(Q8 ? tp_wait_both(full0 + 8 * slot, phase, &sh->abort_flag) : tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag))) {
                         if (lane == 0) atomicOr(status, 4u);
                         sh->abort_flag = 1;
                         stop = true;
@@ -168,10 +203,148 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4), db = da + (TP_A_BYTES >> 4);
                     tp_mma4(d_tmem, da, db, idesc, kb > 0 ? 1u : 0u);
+                    if (Q8) tp_mma4(d_tmem, da, db + (uint64_t)((half * 128) >> 4), idesc, 1u);
                     tp_commit_both(empty0 + 8 * slot);
-                    if (++slot == TP_STAGES) { slot = 0; phase ^= 1u; }
+                    if (++slot == STAGES) { slot = 0; phase ^= 1u; }
                 }
                 tp_commit_both(tc_smem(&sh->tmem_full[ab]));
+            }
+        }
+    } else if (Q8 && warp == TPQ_THREADS / 32 - 1) {
+        // ---------------- Q8_0: TMA producer of the weights' bytes and scales (no kernel writes them: no dependency wait)
+        int slot = 0;
+        uint32_t phase = 1;
+        bool stop = false;
+        for (int tile = pair; tile < n_tiles && !stop; tile += n_pairs) {
+            const int row = tile / n_mt * step + (rank == 0 ? 0 : (swiglu ? a.di : half));
+            for (int kb = 0; kb < nkb; kb += 4) {
+                if (!tc_warp_wait(tc_smem(&sh->g_empty[0]) + 8 * slot, phase, &sh->abort_flag)) {
+                    if (lane == 0) atomicOr(status, 4u);
+                    sh->abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                const uint32_t bar = tc_smem(&sh->g_full[0]) + 8 * slot, dst = tc_smem(raw) + (uint32_t)(slot * TPQ_G_BYTES);
+                tc_warp_expect_tx(bar, (uint32_t)TPQ_G_BYTES);
+                tc_warp_tma_2d(dst, &map_w, kb * TC_BK, row, bar);
+                tc_warp_tma_2d(dst + TPQ_Q_BYTES / 2, &map_w, kb * TC_BK + 128, row, bar);
+                tc_warp_tma_2d(dst + TPQ_Q_BYTES, &map_s, kb * 2, row, bar);
+                if (++slot == TPQ_GROUPS) { slot = 0; phase ^= 1u; }
+            }
+        }
+    } else if (Q8 && warp >= TP_THREADS / 32) {
+        // ---------------- Q8_0: the converting warps work in pairs, one stage of a group each (a row per thread): the fence and the
+        // hand-over of a stage take longer than its arithmetic, and so they run side by side
+        if constexpr (Q8) {
+            const int u = (warp - TP_THREADS / 32) >> 1, row = (tid - TP_THREADS) & (TPQ_ROWS - 1);
+            const uint32_t empty0 = tc_smem(&sh->empty[0]), full0_leader = tp_in_leader(tc_smem(&sh->full[0]));
+            int slot = u, gs = 0;
+            uint32_t phase = 1, g_phase = 0;
+            bool stop = false;
+            for (int tile = pair; tile < n_tiles && !stop; tile += n_pairs)
+                for (int kb = 0; kb < nkb; kb += 4) {
+                    stop = !tc_warp_wait(tc_smem(&sh->g_full[0]) + 8 * gs, g_phase, &sh->abort_flag);
+                    if (stop) break;
+                    const unsigned char *group = raw + (size_t)gs * TPQ_G_BYTES;
+                    const __half2 pair2 = *reinterpret_cast<const __half2 *>(group + TPQ_Q_BYTES + row * 16 + 4 * u);
+                    uint4 q[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        q[c] = *reinterpret_cast<const uint4 *>(group + (u >> 1) * (TPQ_Q_BYTES / 2) + row * 128 + ((((u & 1) * 4 + c) ^ (row & 7)) << 4));
+                    stop = !tc_warp_wait(empty0 + 8 * slot, phase, &sh->abort_flag);
+                    if (stop) break;
+                    unsigned char *line = smem + (size_t)slot * stage_bytes + TP_A_BYTES + row * 128;  // 128-byte swizzle
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t hi[8], lo[8];
+                        tc_q8_split(q[c], c >> 1 ? __high2half2(pair2) : __low2half2(pair2), hi, lo);
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int at = ((c * 2 + k) ^ (row & 7)) << 4;
+                            *reinterpret_cast<uint4 *>(line + at) = make_uint4(hi[4 * k], hi[4 * k + 1], hi[4 * k + 2], hi[4 * k + 3]);
+                            *reinterpret_cast<uint4 *>(line + TPQ_ROWS * 128 + at) = make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(full0_leader + 8 * slot) : "memory");
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&sh->g_empty[0]) + 8 * gs) : "memory");
+                    }
+                    slot += 4;
+                    if (slot >= STAGES) { slot -= STAGES; phase ^= 1u; }
+                    if (++gs == TPQ_GROUPS) { gs = 0; g_phase ^= 1u; }
+                }
+            if (stop) {
+                if (lane == 0) atomicOr(status, 4u);
+                sh->abort_flag = 1;
+            }
+        }
+    } else if (Q8 && warp >= 2) {
+        // ---------------- Q8_0: epilogue.  A thread has one token and 64 outputs (SwiGLU: 32 gates, then their ups): sums over the groups
+        if constexpr (Q8) {
+            const int q = warp & 3, h = (warp - 2) >> 2;
+            const int c_a = swiglu ? h * 32 : h * 64, c_b = swiglu ? TPQ_ROWS + h * 32 : c_a + 32;
+            int ti = 0;
+            bool ok = true;
+            grid_dep_wait();
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+                const int nt = tile / n_mt, mt = tile - nt * n_mt;
+                const int n = mt * 2 * TP_BM + rank * TP_BM + q * 32 + lane;
+                float sum[64];
+#pragma unroll
+                for (int i = 0; i < 64; ++i) sum[i] = 0.f;
+                for (int kb = 0; kb < nkb && ok; kb += 4, ++ti) {
+                    const int ab = ti & 1;
+                    ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * TP_COLS);
+#pragma unroll
+                    for (int c = 0; c < 64; c += 16) {
+                        uint32_t r[16];
+                        tc_ld16(acc + (uint32_t)(c < 32 ? c_a + c : c_b + c - 32), r);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(r[i]);
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
+                }
+                if (!ok) break;
+                if (n >= a.n_tok) continue;
+                if (swiglu) {
+#pragma unroll
+                    for (int c = 0; c < 32; c += 8) {
+                        const int first = nt * step + c_a + c;
+                        if (first + 8 > a.di) continue;
+                        TcPre pre;
+                        tc_q8_mend(a, n, first, sum + c);
+                        tc_q8_mend(a, n, a.di + first, sum + 32 + c);
+                        tc_finish<T>(a, n, first, sum + c, sum + 32 + c, pre);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 64; c += 16) {
+                        const int first = nt * step + c_a + c;
+                        TcPre pre[2];
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+                            if (first + 8 * k + 8 <= a.out) tc_prefetch<T>(a, n, first + 8 * k, pre[k]);
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            if (first + 8 * k + 8 > a.out) continue;
+                            tc_q8_mend(a, n, first + 8 * k, sum + c + 8 * k);
+                            tc_finish<T>(a, n, first + 8 * k, sum + c + 8 * k, sum + c + 8 * k, pre[k]);
+                        }
+                    }
+                }
+            }
+            if (!ok) {
+                if (lane == 0) atomicOr(status, 4u);
+                sh->abort_flag = 1;
             }
         }
     } else if (warp >= 2) {
@@ -246,7 +419,8 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
 
 // ------------------------------------------------------------------ host side
 
-static size_t tp_smem_bytes() { return 1024 + (size_t)TP_STAGES * (TP_A_BYTES + TP_COLS / 2 * 128) + sizeof(TpShared); }
+template <bool Q8>
+static size_t tp_smem_bytes() { return 1024 + (size_t)(Q8 ? TPQ_STAGES * (TP_A_BYTES + 2 * TPQ_ROWS * 128) + TPQ_GROUPS * TPQ_G_BYTES : TP_STAGES * (TP_A_BYTES + TP_COLS / 2 * 128)) + sizeof(TpShared); }
 
 // Weight rows of a tile: the time of a stage goes with the rows that both operands bring (0.29 us for 256 + 128, 0.43 us for
 // 256 + 256), so the fewest rows that the busiest pair loads.
@@ -263,13 +437,13 @@ static int tp_tile(int n_mt, int rows, int pairs) {
 bool gemm_pair_takes(const GemvArgs &a) {
     const int min = tuning().tc_pair_min;
     if (min <= 0 || a.n_tok < min || a.tiles || a.push.n || !tc_vec(a)) return false;
-    if (min == 1) return true;
+    if (min == 1 || a.w_q8) return true;  // (Q8_0 weights have passes of 64 tokens otherwise)
     const int rows = a.epilogue == EPI_SWIGLU ? 2 * a.di : a.out, n_mt = (a.n_tok + 2 * TP_BM - 1) / (2 * TP_BM), pairs = sm_count() / 2;
     const int NT = tp_tile(n_mt, rows, pairs);
     return 2 * n_mt * ((rows + NT - 1) / NT) > pairs;
 }
 
-template <class T>
+template <class T, bool Q8>
 static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, bool dry) {
     static std::mutex mu;
     static std::map<int, bool> done;
@@ -278,7 +452,7 @@ static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!done[dev]) {
-            LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes()));
+            LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<T, Q8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes<Q8>()));
             done[dev] = true;
         }
     }
@@ -286,28 +460,30 @@ static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32
     const int pairs = sm_count() / 2;
     const int n_mt = (a.n_tok + 2 * TP_BM - 1) / (2 * TP_BM);
     const int outs = a.epilogue == EPI_SWIGLU ? a.di : a.out, per = a.epilogue == EPI_SWIGLU ? 2 : 1;
-    const int NT = tp_tile(n_mt, outs * per, pairs);
+    const int NT = Q8 ? 2 * TPQ_ROWS : tp_tile(n_mt, outs * per, pairs);
     const int n_nt = (outs * per + NT - 1) / NT;
-    CUtensorMap mw, mx;
-    int rc = tc_make_map(&mw, a.w, dt, (uint64_t)a.out, (uint64_t)a.in, (uint64_t)a.in, (uint32_t)NT / 2);
+    CUtensorMap mw, ms, mx;
+    int rc = Q8 ? tc_make_q8_maps(&mw, &ms, a.w, a.w_scales, (uint64_t)a.out, (uint64_t)a.in) : tc_make_map(&mw, a.w, dt, (uint64_t)a.out, (uint64_t)a.in, (uint64_t)a.in, (uint32_t)NT / 2);
     if (!rc) rc = tc_make_map(&mx, a.x, dt, (uint64_t)a.n_tok, (uint64_t)a.in, (uint64_t)a.stride_x, TP_BM);
     if (rc) return rc;
     const uint32_t fmt = dt == LCU_BF16 ? 1u : 0u;
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(2 * TP_BM >> 4) << 24);
     const int tiles = n_mt * n_nt;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);
-    LCU_CHECK_CUDA(launch_kernel(gemm_pair_kernel<T>, dim3(grid), dim3(TP_THREADS), tp_smem_bytes(), s, pdl, a, mw, mx, NT, n_mt, tiles, idesc, status));
+    LCU_CHECK_CUDA(launch_kernel(gemm_pair_kernel<T, Q8>, dim3(grid), dim3(Q8 ? TPQ_THREADS : TP_THREADS), tp_smem_bytes<Q8>(), s, pdl, a, mw, Q8 ? ms : mw, mx, NT, n_mt, tiles, idesc, status));
     g_linear_last_ctas = grid;
     return LCU_OK;
 }
 
 int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status) {
-    return dt == LCU_F16 ? tp_launch<__half>(a, dt, s, pdl, status, false) : tp_launch<__nv_bfloat16>(a, dt, s, pdl, status, false);
+    if (a.w_q8) return tp_launch<__half, true>(a, dt, s, pdl, status, false);
+    return dt == LCU_F16 ? tp_launch<__half, false>(a, dt, s, pdl, status, false) : tp_launch<__nv_bfloat16, false>(a, dt, s, pdl, status, false);
 }
 
-int gemm_pair_warm(int dt) {
+int gemm_pair_warm(int dt, bool q8) {
     GemvArgs a{};
-    return dt == LCU_F16 ? tp_launch<__half>(a, dt, nullptr, false, nullptr, true) : tp_launch<__nv_bfloat16>(a, dt, nullptr, false, nullptr, true);
+    if (q8) return tp_launch<__half, true>(a, dt, nullptr, false, nullptr, true);
+    return dt == LCU_F16 ? tp_launch<__half, false>(a, dt, nullptr, false, nullptr, true) : tp_launch<__nv_bfloat16, false>(a, dt, nullptr, false, nullptr, true);
 }
 
 }  // namespace lcu

@@ -34,8 +34,27 @@ constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;
 
 constexpr int TC_MAX_STAGES = 12;
 
+// Q8_0 weights: 8 more warps turn a unit's weights into f16 pairs in tensor memory, from where the MMA takes them as its A operand
+// (lane = row); through shared memory they would cost it four times the bytes that HBM delivers.
+constexpr int TQ_THREADS = TC_THREADS + 256;
+constexpr int TQ_W_BYTES = TC_BM * TQ_K, TQ_S_BYTES = TC_BM * (TQ_K / 32) * 2;
+constexpr int TQ_RING = 6, TQ_COL = 128;  // K blocks in tensor memory, the first one's column
+template <bool Q8> constexpr int tc_unit_w_bytes() { return Q8 ? TQ_W_BYTES + TQ_S_BYTES : TC_A_BYTES; }
+template <bool Q8> __host__ __device__ constexpr int tc_unit_bytes(int N) { return Q8 ? TQ_W_BYTES + TQ_S_BYTES + N * 2 * TQ_K : TC_A_BYTES + N * 128; }
+
+__device__ __forceinline__ void tq_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred e, p;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+                 " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tq_st16(uint32_t taddr, const uint32_t *r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
 struct TcShared {
-    unsigned long long full[TC_MAX_STAGES], empty[TC_MAX_STAGES], tmem_full[2], tmem_empty[2];
+    unsigned long long full[TC_MAX_STAGES], empty[TC_MAX_STAGES], tmem_full[2], tmem_empty[2], a_full[TQ_RING], a_empty[TQ_RING];
     uint32_t tmem_base;
     int abort_flag;
     int last;
@@ -44,25 +63,29 @@ struct TcShared {
 // Persistent: grid = min(tiles, SMs); a tile is (row block of 128 rows = 64 pairs, K split); CTA c takes
 // tiles c, c + grid, ...  The shared-memory ring keeps running across tiles and the accumulator is
 // double-buffered in TMEM, so the epilogue of one tile overlaps the loads and MMAs of the next.
-// block = 6 warps: TMA producer, MMA issuer, 4 epilogue warps.
-template <class T>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+// block = 6 warps: TMA producer, MMA issuer, 4 epilogue warps; Q8_0: 8 warps more.
+// Q8_0: a unit is 256 K elements of a row block with their scales, in four K blocks of 64.  The converting warps work in two groups
+// that take the K blocks in turns (a row per thread) and hand them to the MMA through a ring of six in tensor memory, 64 columns
+// each: one group's waits run under the other's arithmetic, which is about 180 cycles a K block against 370 that its bytes take.
+// 8B shape, 16 sequences: 5.13 -> 3.87 ms per round against the mma.sync kernel (28672 x 4096 in 34 us, its bytes 20).
+template <class T, bool Q8>
+__global__ void __launch_bounds__(Q8 ? TQ_THREADS : TC_THREADS, 1)
+gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_x,
                int n_pairs, int N, int n_stages, int units_per_cta, int max_seg, int vec, uint32_t idesc, float *ws,
                unsigned *tickets, uint32_t *status) {
     extern __shared__ unsigned char smem_raw[];
     // 1024-byte alignment: the 128-byte swizzle pattern repeats every 8 rows = 1024 bytes
     unsigned char *smem = smem_raw + ((1024u - (tc_smem(smem_raw) & 1023u)) & 1023u);
-    const int stage_bytes = TC_A_BYTES + N * 128;
+    const int stage_bytes = tc_unit_bytes<Q8>(N);
     float *stg = reinterpret_cast<float *>(smem + (size_t)n_stages * stage_bytes);  // [128][N + 1]
     TcShared *sh = reinterpret_cast<TcShared *>(reinterpret_cast<unsigned char *>(stg) + (size_t)TC_BM * (N + 1) * 4);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (a.pdl_trigger == 0) grid_dep_launch();
-    const int nkb = a.in / TC_BK;  // K blocks of a whole row block
+    const int nkb = a.in / (Q8 ? TQ_K : TC_BK);  // K blocks (Q8_0: units) of a whole row block
     const bool swiglu = a.epilogue == EPI_SWIGLU;
-    const int acc_cols = N < 32 ? 32 : N;      // TMEM columns of one accumulator
-    const int tm_cols = 2 * acc_cols;          // two accumulators
+    const int acc_cols = N < 32 ? 32 : (N == 48 ? 64 : N);  // TMEM columns of one accumulator
+    const int tm_cols = Q8 ? 512 : 2 * acc_cols;            // two accumulators (Q8_0: and the weights)
     const int n_rb = (n_pairs + 63) / 64;
     // work units = (row block, K block) pairs in row-block-major order; this CTA owns a contiguous range and
     // walks it as segments that end at row-block boundaries (stream-K)
@@ -73,11 +96,15 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
     if (tid == 0) {
         for (int i = 0; i < n_stages; ++i) {
             tc_mbar_init(tc_smem(&sh->full[i]), 1);
-            tc_mbar_init(tc_smem(&sh->empty[i]), 1);
+            tc_mbar_init(tc_smem(&sh->empty[i]), Q8 ? 9 : 1);  // Q8_0: the MMAs and the 8 converting warps
         }
         for (int i = 0; i < 2; ++i) {
             tc_mbar_init(tc_smem(&sh->tmem_full[i]), 1);
-            tc_mbar_init(tc_smem(&sh->tmem_empty[i]), 1);
+            tc_mbar_init(tc_smem(&sh->tmem_empty[i]), Q8 ? 4 : 1);
+        }
+        for (int i = 0; Q8 && i < TQ_RING; ++i) {
+            tc_mbar_init(tc_smem(&sh->a_full[i]), 4);
+            tc_mbar_init(tc_smem(&sh->a_empty[i]), 1);
         }
         sh->abort_flag = 0;
         sh->last = 0;
@@ -103,11 +130,21 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
         auto weights = [&](int slot, int kb, int rb) {
             const uint32_t bar = full0 + 8 * slot, dst = smem0 + (uint32_t)(slot * stage_bytes);
             tc_warp_expect_tx(bar, (uint32_t)stage_bytes);
-            tc_warp_tma_2d(dst, &map_w, kb * TC_BK, rb * row_step, bar);
-            tc_warp_tma_2d(dst + TC_A_BYTES / 2, &map_w, kb * TC_BK, second + rb * row_step, bar);
+            if constexpr (Q8) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)  // [2 x 128 K][2 x 64 rows], then the scales [2 x 64 rows]
+                    tc_warp_tma_2d(dst + i * (TQ_W_BYTES / 4), &map_w, kb * TQ_K + (i >> 1) * 128, (i & 1) * second + rb * row_step, bar);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    tc_warp_tma_2d(dst + TQ_W_BYTES + i * (TQ_S_BYTES / 2), &map_s, kb * (TQ_K / 32), i * second + rb * row_step, bar);
+            } else {
+                tc_warp_tma_2d(dst, &map_w, kb * TC_BK, rb * row_step, bar);
+                tc_warp_tma_2d(dst + TC_A_BYTES / 2, &map_w, kb * TC_BK, second + rb * row_step, bar);
+            }
         };
         auto acts = [&](int slot, int kb) {
-            tc_warp_tma_2d(smem0 + (uint32_t)(slot * stage_bytes + TC_A_BYTES), &map_x, kb * TC_BK, 0, full0 + 8 * slot);
+            const uint32_t dst = smem0 + (uint32_t)(slot * stage_bytes + tc_unit_w_bytes<Q8>());
+            for (int i = 0; i < (Q8 ? 4 : 1); ++i) tc_warp_tma_2d(dst + (uint32_t)(i * N * 128), &map_x, (kb * (Q8 ? 4 : 1) + i) * TC_BK, 0, full0 + 8 * slot);
         };
         // The weights do not depend on the previous kernel: when this launch was allowed to start early
         // (programmatic dependent launch) the first ring of weight tiles is already streaming while the predecessor
@@ -141,8 +178,10 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
         const uint64_t desc0 = tc_desc(tc_smem(smem));
         int slot = 0, ti = 0, kb0 = u_begin % nkb;
         uint32_t phase = 0;
+        [[maybe_unused]] int at = 0;  // Q8_0: the ring in tensor memory
+        [[maybe_unused]] uint32_t at_phase = 0;
         for (int u = u_begin; u < u_end && !sh->abort_flag; ++ti) {
-            const int kb1 = min(nkb, kb0 + (u_end - u));
+            const int kb1 = Q8 ? kb0 + 1 : min(nkb, kb0 + (u_end - u));  // Q8_0: every unit has an accumulator of its own
             const int ab = ti & 1;
             // the epilogue must have drained this accumulator (two tiles ago)
             if (!tc_warp_wait(tc_smem(&sh->tmem_empty[ab]), ((uint32_t)(ti >> 1) & 1u) ^ 1u, &sh->abort_flag)) {
@@ -160,13 +199,86 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4);
-                tc_warp_mma4(d_tmem, da, da + (TC_A_BYTES >> 4), idesc, kb > kb0 ? 1u : 0u);
+                if constexpr (Q8) {
+                    bool ok = true;
+                    for (int b = 0; b < 4; ++b) {
+                        ok = tc_warp_wait(tc_smem(&sh->a_full[0]) + 8 * at, at_phase, &sh->abort_flag);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint64_t db = da + (uint64_t)((tc_unit_w_bytes<Q8>() + b * N * 128) >> 4);
+                        const uint32_t ta = tmem + TQ_COL + 64 * at;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            tq_mma(d_tmem, ta + 8 * k, db + 2 * k, idesc, kb > kb0 || b > 0 || k > 0);
+                            tq_mma(d_tmem, ta + 32 + 8 * k, db + 2 * k, idesc, 1u);
+                        }
+                        tc_warp_commit(tc_smem(&sh->a_empty[0]) + 8 * at);
+                        if (++at == TQ_RING) { at = 0; at_phase ^= 1u; }
+                    }
+                    if (!ok) {
+                        if (lane == 0) atomicOr(status, 4u);
+                        sh->abort_flag = 1;
+                        break;
+                    }
+                } else {
+                    tc_warp_mma4(d_tmem, da, da + (TC_A_BYTES >> 4), idesc, kb > kb0 ? 1u : 0u);
+                }
                 tc_warp_commit(empty0 + 8 * slot);  // the stage is free once these MMAs have read it
                 if (++slot == n_stages) { slot = 0; phase ^= 1u; }
             }
             tc_warp_commit(tc_smem(&sh->tmem_full[ab]));     // accumulator complete
             u += kb1 - kb0;
-            kb0 = 0;
+            kb0 = Q8 && kb1 < nkb ? kb1 : 0;
+        }
+    } else if (Q8 && warp >= TC_THREADS / 32) {
+        // ---------------- Q8_0: a thread turns a row's 64 K elements (two quantisation blocks) into f16 pairs
+        if constexpr (Q8) {
+            const int q = warp & 3, grp = (warp - TC_THREADS / 32) >> 2, row = q * 32 + lane;  // a warp may only touch TMEM lanes [32 q, 32 q + 32)
+            const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + TQ_COL;
+            int slot = 0, at = grp;  // this group's places: grp, grp + 2, grp + 4
+            uint32_t phase = 0, at_phase = 1;
+            bool ok = true;
+            for (int u = u_begin; u < u_end && ok; ++u) {
+                ok = tc_warp_wait(tc_smem(&sh->full[0]) + 8 * slot, phase, &sh->abort_flag);
+                if (!ok) break;
+                const unsigned char *unit = smem + (size_t)slot * stage_bytes;
+                const uint4 sc = *reinterpret_cast<const uint4 *>(unit + TQ_W_BYTES + row * 16);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t sw = i ? (grp ? sc.w : sc.z) : (grp ? sc.y : sc.x);
+                    const unsigned char *line = unit + i * (TQ_W_BYTES / 2) + row * 128;  // 128-byte swizzle
+                    uint4 raw[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) raw[c] = *reinterpret_cast<const uint4 *>(line + (((grp * 4 + c) ^ (row & 7)) << 4));
+                    ok = tc_warp_wait(tc_smem(&sh->a_empty[0]) + 8 * at, at_phase, &sh->abort_flag);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const __half2 pair = *reinterpret_cast<const __half2 *>(&sw);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t hi[16], lo[16];
+                        const __half2 s2 = h ? __high2half2(pair) : __low2half2(pair);
+                        tc_q8_split(raw[2 * h], s2, hi, lo);
+                        tc_q8_split(raw[2 * h + 1], s2, hi + 8, lo + 8);
+                        tq_st16(ta + 64 * at + 16 * h, hi);
+                        tq_st16(ta + 64 * at + 32 + 16 * h, lo);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&sh->a_full[0]) + 8 * at) : "memory");
+                        if (i == 1) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&sh->empty[0]) + 8 * slot) : "memory");
+                    }
+                    at += 2;
+                    if (at >= TQ_RING) { at = grp; at_phase ^= 1u; }
+                }
+                if (++slot == n_stages) { slot = 0; phase ^= 1u; }
+            }
+            if (!ok) {
+                if (lane == 0) atomicOr(status, 4u);
+                sh->abort_flag = 1;
+            }
         }
     } else if (warp >= 2) {
         // ---------------- epilogue warps: TMEM -> registers -> shared staging -> fused epilogue
@@ -174,6 +286,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
         const int q = warp & 3;                      // a warp may only touch TMEM lanes [32q, 32q + 32)
         const int row = q * 32 + lane;
         int ti = 0;
+        [[maybe_unused]] int tu = 0;  // Q8_0: units taken
         for (int u = u_begin; u < u_end; ++ti) {
             const int rb = u / nkb, kb0 = u - rb * nkb;
             const int kb1 = min(nkb, kb0 + (u_end - u));
@@ -183,13 +296,45 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             const int first_cta = (rb * nkb) / units_per_cta, last_cta = (rb * nkb + nkb - 1) / units_per_cta;
             const int n_seg = last_cta - first_cta + 1, seg = (int)blockIdx.x - first_cta;
             const int ab = ti & 1;
-            bool ok = tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag);
+            bool ok;
+            [[maybe_unused]] float sum[Q8 ? 64 : 1];
+            if constexpr (Q8) {
+                // the tensor pipe cuts a sum off where it would have to round it, which thousands of products in a row show: units are
+                // added up here, rounded
+#pragma unroll
+                for (int i = 0; i < 64; ++i) sum[i] = 0.f;
+                ok = true;
+                for (int kb = kb0; kb < kb1 && ok; ++kb, ++tu) {
+                    const int ub = tu & 1;
+                    ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ub]), (uint32_t)(tu >> 1) & 1u, &sh->abort_flag));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int c0 = 0; c0 < 64; c0 += 16)
+                        if (c0 < N) {
+                            uint32_t r[16];
+                            tc_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ub * acc_cols + c0), r);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) sum[c0 + i] += __uint_as_float(r[i]);
+                        }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&sh->tmem_empty[ub])) : "memory");
+                }
+            } else {
+                ok = tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag);
+            }
             if (!ok) {
                 atomicOr(status, 4u);
                 sh->abort_flag = 1;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (ok) {
+            if constexpr (Q8) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i)
+                    if (i < N) stg[row * (N + 1) + i] = sum[i];
+            } else if (ok) {
                 for (int c0 = 0; c0 < N; c0 += 16) {
                     uint32_t r[16];
                     tc_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * acc_cols + c0), r);
@@ -204,7 +349,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             uint32_t all_ok;
             asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, 2, 128, p;\n selp.u32 %0, 1, 0, q;\n}"
                          : "=r"(all_ok) : "r"((uint32_t)ok) : "memory");
-            if (et == 0) {  // the accumulator may be overwritten from here on
+            if (!Q8 && et == 0) {  // the accumulator may be overwritten from here on
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&sh->tmem_empty[ab])) : "memory");
             }
             if (!all_ok) break;
@@ -230,6 +375,10 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                         v[i] = stg[(8 * c + i) * (N + 1) + n];
                         u[i] = swiglu ? stg[(64 + 8 * c + i) * (N + 1) + n] : 0.f;
                     }
+                    if constexpr (Q8) {
+                        tc_q8_mend(a, n, first, v);
+                        if (swiglu) tc_q8_mend(a, n, a.di + first, u);
+                    }
                     tc_finish<T>(a, n, first, v, u, pre[cnt]);
                 }
             } else if (whole) {
@@ -238,7 +387,12 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                     int p = rb * 64 + j;
                     if (p >= n_pairs || n >= a.n_tok) continue;
                     int ra = swiglu ? j : 2 * j, rb2 = swiglu ? 64 + j : 2 * j + 1;
-                    gemv_epilogue<T>(a, p, n, stg[ra * (N + 1) + n], stg[rb2 * (N + 1) + n]);
+                    float va = stg[ra * (N + 1) + n], vb = stg[rb2 * (N + 1) + n];
+                    if constexpr (Q8) {
+                        if (!(fabsf(va) < INFINITY)) va = tc_q8_dot(a, n, swiglu ? p : 2 * p);
+                        if (!(fabsf(vb) < INFINITY)) vb = tc_q8_dot(a, n, swiglu ? a.di + p : 2 * p + 1);
+                    }
+                    gemv_epilogue<T>(a, p, n, va, vb);
                 }
             } else {
                 // the row block is shared (the host only cuts row blocks when the vector epilogue applies).  Partial
@@ -268,39 +422,35 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                     __threadfence();
                     // Merge of the segments' partial sums.  A partial row lives in the L2 slice of whichever SM wrote
                     // it and one dependent round trip costs more than a microsecond here, so the loads of up to 6
-                    // segments for TWO rows of 8 floats are all issued before the first add (96 registers of loads in
-                    // flight per thread; the epilogue warps have registers to spare), the adds then run in K order.
+                    // segments (Q8_0, whose threads have fewer registers: 3) for TWO rows of 8 floats are all issued before the
+                    // first add, the adds then run in K order.
                     // Measured on a 6-segment merge of a 128 x 32 tile: 11 us with one segment after the other.
+                    constexpr int MB = Q8 ? 3 : 6;
                     const size_t seg_stride = (size_t)N * TC_BM;
                     auto merge2 = [&](const float *r0, const float *r1, float o0[8], float o1[8]) {
-                        float4 b0[12], b1[12];
-#pragma unroll
-                        for (int s2 = 0; s2 < 6; ++s2) {
-                            if (s2 < n_seg) {
-                                b0[2 * s2] = __ldcg(reinterpret_cast<const float4 *>(r0 + s2 * seg_stride));
-                                b0[2 * s2 + 1] = __ldcg(reinterpret_cast<const float4 *>(r0 + s2 * seg_stride + 4));
-                                b1[2 * s2] = __ldcg(reinterpret_cast<const float4 *>(r1 + s2 * seg_stride));
-                                b1[2 * s2 + 1] = __ldcg(reinterpret_cast<const float4 *>(r1 + s2 * seg_stride + 4));
-                            }
-                        }
 #pragma unroll
                         for (int i = 0; i < 8; ++i) o0[i] = o1[i] = 0.f;
+                        for (int base = 0; base < n_seg; base += MB) {  // (more than 6 CTAs on one row block: small launches only)
+                            float4 b0[2 * MB], b1[2 * MB];
 #pragma unroll
-                        for (int s2 = 0; s2 < 6; ++s2) {
-                            if (s2 < n_seg) {
-                                o0[0] += b0[2 * s2].x; o0[1] += b0[2 * s2].y; o0[2] += b0[2 * s2].z; o0[3] += b0[2 * s2].w;
-                                o0[4] += b0[2 * s2 + 1].x; o0[5] += b0[2 * s2 + 1].y; o0[6] += b0[2 * s2 + 1].z; o0[7] += b0[2 * s2 + 1].w;
-                                o1[0] += b1[2 * s2].x; o1[1] += b1[2 * s2].y; o1[2] += b1[2 * s2].z; o1[3] += b1[2 * s2].w;
-                                o1[4] += b1[2 * s2 + 1].x; o1[5] += b1[2 * s2 + 1].y; o1[6] += b1[2 * s2 + 1].z; o1[7] += b1[2 * s2 + 1].w;
+                            for (int s2 = 0; s2 < MB; ++s2) {
+                                if (base + s2 < n_seg) {
+                                    const size_t off = (size_t)(base + s2) * seg_stride;
+                                    b0[2 * s2] = __ldcg(reinterpret_cast<const float4 *>(r0 + off));
+                                    b0[2 * s2 + 1] = __ldcg(reinterpret_cast<const float4 *>(r0 + off + 4));
+                                    b1[2 * s2] = __ldcg(reinterpret_cast<const float4 *>(r1 + off));
+                                    b1[2 * s2 + 1] = __ldcg(reinterpret_cast<const float4 *>(r1 + off + 4));
+                                }
                             }
-                        }
-                        for (int s2 = 6; s2 < n_seg; ++s2) {  // more than 6 CTAs on one row block: small launches only
-                            const float4 a0 = __ldcg(reinterpret_cast<const float4 *>(r0 + s2 * seg_stride));
-                            const float4 a1 = __ldcg(reinterpret_cast<const float4 *>(r0 + s2 * seg_stride + 4));
-                            const float4 c0 = __ldcg(reinterpret_cast<const float4 *>(r1 + s2 * seg_stride));
-                            const float4 c1 = __ldcg(reinterpret_cast<const float4 *>(r1 + s2 * seg_stride + 4));
-                            o0[0] += a0.x; o0[1] += a0.y; o0[2] += a0.z; o0[3] += a0.w; o0[4] += a1.x; o0[5] += a1.y; o0[6] += a1.z; o0[7] += a1.w;
-                            o1[0] += c0.x; o1[1] += c0.y; o1[2] += c0.z; o1[3] += c0.w; o1[4] += c1.x; o1[5] += c1.y; o1[6] += c1.z; o1[7] += c1.w;
+#pragma unroll
+                            for (int s2 = 0; s2 < MB; ++s2) {
+                                if (base + s2 < n_seg) {
+                                    o0[0] += b0[2 * s2].x; o0[1] += b0[2 * s2].y; o0[2] += b0[2 * s2].z; o0[3] += b0[2 * s2].w;
+                                    o0[4] += b0[2 * s2 + 1].x; o0[5] += b0[2 * s2 + 1].y; o0[6] += b0[2 * s2 + 1].z; o0[7] += b0[2 * s2 + 1].w;
+                                    o1[0] += b1[2 * s2].x; o1[1] += b1[2 * s2].y; o1[2] += b1[2 * s2].z; o1[3] += b1[2 * s2].w;
+                                    o1[4] += b1[2 * s2 + 1].x; o1[5] += b1[2 * s2 + 1].y; o1[6] += b1[2 * s2 + 1].z; o1[7] += b1[2 * s2 + 1].w;
+                                }
+                            }
                         }
                     };
                     const float *tile0 = ws + (size_t)rb * max_seg * seg_stride;
@@ -314,6 +464,10 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                             float g8[8], u8[8];
                             const float *r = tile0 + (size_t)n * TC_BM + 8 * c;
                             merge2(r, r + 64, g8, u8);
+                            if constexpr (Q8) {
+                                tc_q8_mend(a, n, first, g8);
+                                tc_q8_mend(a, n, a.di + first, u8);
+                            }
                             TcPre pre;
                             tc_finish<T>(a, n, first, g8, u8, pre);
                         }
@@ -332,6 +486,10 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                             const float *r0 = tile0 + (size_t)(v0 ? n0 : n1) * TC_BM + 8 * c;
                             const float *r1 = tile0 + (size_t)(v1 ? n1 : n0) * TC_BM + 8 * c;
                             merge2(r0, r1, o0, o1);
+                            if constexpr (Q8) {
+                                if (v0) tc_q8_mend(a, n0, first, o0);
+                                if (v1) tc_q8_mend(a, n1, first, o1);
+                            }
                             if (v0) tc_finish<T>(a, n0, first, o0, zero8, pre0);
                             if (v1) tc_finish<T>(a, n1, first, o1, zero8, pre1);
                         }
@@ -569,10 +727,11 @@ void gemm_tc_set_scratch(void *ws, size_t ws_bytes, unsigned *tickets, int n_tic
     g_tc_status = status;
 }
 
-bool gemm_tc_supported(int in, int w_q8) { return !w_q8 && in >= TC_BK && in % TC_BK == 0 && tc_encode_fn() != nullptr; }
+bool gemm_tc_supported(int in, int w_q8) { return in >= TC_BK && in % (w_q8 ? TQ_K : TC_BK) == 0 && tc_encode_fn() != nullptr; }
 
+template <bool Q8>
 static size_t tc_smem_bytes(int N, int stages) {
-    return 1024 + (size_t)stages * (TC_A_BYTES + N * 128) + (size_t)TC_BM * (N + 1) * 4 + sizeof(TcShared) + 64;
+    return 1024 + (size_t)stages * tc_unit_bytes<Q8>(N) + (size_t)TC_BM * (N + 1) * 4 + sizeof(TcShared) + 64;
 }
 
 // Clusters of ks CTAs of the cluster form that run at once on the current device (0: unknown, not possible).
@@ -603,13 +762,20 @@ static int tck_clusters(int ks, size_t smem) {
     return cache[key] = n;
 }
 
-template <class T>
+// Tokens of a launch: the MMA's N.  Q8_0 launches take 64 at most (the ring's units are large).
+template <bool Q8>
+static int tc_columns(const GemvArgs &a) {
+    if (Q8) return a.n_tok <= 16 ? 16 : (a.n_tok <= 32 ? 32 : (a.n_tok <= 48 ? 48 : 64));
+    return a.tiles ? a.tile_rows : a.n_tok <= 16 ? 16 : (a.n_tok <= 32 ? 32 : (a.n_tok <= 64 ? 64 : (a.n_tok <= 128 ? 128 : 256)));
+}
+
+template <class T, bool Q8>
 static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool dry) {
-    auto kernel = gemm_tc_kernel<T>;
-    const int N = a.tiles ? a.tile_rows : a.n_tok <= 16 ? 16 : (a.n_tok <= 32 ? 32 : (a.n_tok <= 64 ? 64 : (a.n_tok <= 128 ? 128 : 256)));
+    auto kernel = gemm_tc_kernel<T, Q8>;
+    const int N = tc_columns<Q8>(a);
     int stages = 8;
-    while (stages > 2 && tc_smem_bytes(N, stages) > (size_t)227 * 1024) --stages;
-    const size_t smem = tc_smem_bytes(N, stages);
+    while (stages > 2 && tc_smem_bytes<Q8>(N, stages) > (size_t)227 * 1024) --stages;
+    const size_t smem = tc_smem_bytes<Q8>(N, stages);
     static std::mutex mu;
     static std::map<int, uint32_t *> done;  // device -> fallback status word (also marks the attribute as set)
     int dev = 0;
@@ -620,19 +786,19 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
         auto it = done.find(dev);
         if (it == done.end()) {
             LCU_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-            LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_tck_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            if (!Q8) LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_tck_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
             void *p = nullptr;
             LCU_CHECK_CUDA(cudaGetSymbolAddress(&p, g_tc_fallback_status));
             it = done.emplace(dev, reinterpret_cast<uint32_t *>(p)).first;
         }
         if (!status) status = it->second;
     }
-    if (dry) return gemm_pair_warm(dt);
+    if (dry) return gemm_pair_warm(dt, Q8);
     if (gemm_pair_takes(a)) return gemm_pair_launch(a, dt, s, pdl, status);
     const int n_pairs = a.out / 2;
     const int sms = sm_count();
     const uint32_t fmt = dt == LCU_BF16 ? 1u : 0u;
-    CUtensorMap mw, mx;
+    CUtensorMap mw, ms, mx;
     int rc;
     // 16-byte epilogue accesses need aligned, 8-divisible outputs
     bool vec_ok = a.stride_y % 8 == 0 && ((uintptr_t)a.y % 16) == 0 && (a.epilogue == EPI_SWIGLU ? a.di % 8 == 0 : a.out % 8 == 0);
@@ -642,14 +808,33 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
                  ((uintptr_t)a.sin_t % 16) == 0 && ((uintptr_t)a.cos_t % 16) == 0;
     const int vec = vec_ok ? 1 : 0;
     LCU_REQUIRE(vec || a.epilogue < EPI_STORE_F32, "gemm_tc: epilogue %d needs rows of a multiple of 8 outputs", a.epilogue);
+    if ((N > 64 && !vec) || (Q8 && a.n_tok > 64)) {
+        // the 16-byte epilogue does not apply to this shape, or Q8_0 weights: 64-token passes of the general form
+        for (int t0 = 0; t0 < a.n_tok; t0 += 64) {
+            GemvArgs b = a;
+            b.n_tok = a.n_tok - t0 < 64 ? a.n_tok - t0 : 64;
+            b.x = reinterpret_cast<const unsigned char *>(a.x) + (size_t)t0 * a.stride_x * 2;
+            b.y = reinterpret_cast<unsigned char *>(a.y) + (size_t)t0 * a.stride_y * 2;  // 16-bit outputs only (f32 ones have the 16-byte epilogue)
+            if (a.res) b.res = reinterpret_cast<const unsigned char *>(a.res) + (size_t)t0 * a.stride_res * 2;
+            if (a.pos) { b.pos = a.pos + t0; b.tok_seq = a.tok_seq + t0; }
+            int rc2 = tc_launch_t<T, Q8>(b, dt, s, pdl, dry);
+            if (rc2) return rc2;
+        }
+        return LCU_OK;
+    }
     // ---- weight rows on M (any output shape; row blocks of 128)
-    rc = tc_make_map(&mw, a.w, dt, (uint64_t)a.out * (a.tiles ? a.groups : 1), (uint64_t)a.in, (uint64_t)a.in, 64);
+    if constexpr (Q8) {
+        rc = tc_make_q8_maps(&mw, &ms, a.w, a.w_scales, (uint64_t)a.out, (uint64_t)a.in);
+    } else {
+        rc = tc_make_map(&mw, a.w, dt, (uint64_t)a.out * (a.tiles ? a.groups : 1), (uint64_t)a.in, (uint64_t)a.in, 64);
+        ms = mw;
+    }
     if (rc) return rc;
     // the activation map has exactly n_tok rows: the rest of the N-row box is out of bounds and zero-filled
     rc = tc_make_map(&mx, a.x, dt, (uint64_t)a.n_tok, (uint64_t)a.in, (uint64_t)a.stride_x, (uint32_t)N);
     if (rc) return rc;
     // ---- few row blocks: the CTAs of a row block form a cluster and merge through distributed shared memory
-    {
+    if constexpr (!Q8) {
         // tuning 1: where it costs less than the stream-K split, 2: wherever it applies, 0: never
         const int cluster_mode = tuning().tc_cluster;
         const int n_rb_c = (n_pairs + 63) / 64, nkb_c = a.in / TC_BK;
@@ -700,27 +885,13 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
             return LCU_OK;
         }
     }
-    if (N > 64) {
-        // the 16-byte epilogue does not apply to this shape: 64-token passes of the general form
-        for (int t0 = 0; t0 < a.n_tok; t0 += 64) {
-            GemvArgs b = a;
-            b.n_tok = a.n_tok - t0 < 64 ? a.n_tok - t0 : 64;
-            b.x = reinterpret_cast<const unsigned char *>(a.x) + (size_t)t0 * a.stride_x * 2;
-            b.y = reinterpret_cast<unsigned char *>(a.y) + (size_t)t0 * a.stride_y * 2;  // 16-bit outputs only (f32 ones have the 16-byte epilogue)
-            if (a.res) b.res = reinterpret_cast<const unsigned char *>(a.res) + (size_t)t0 * a.stride_res * 2;
-            if (a.pos) { b.pos = a.pos + t0; b.tok_seq = a.tok_seq + t0; }
-            int rc2 = tc_launch_t<T>(b, dt, s, pdl, dry);
-            if (rc2) return rc2;
-        }
-        return LCU_OK;
-    }
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
     // Work split (stream-K): the (row block, K block) units are dealt to the SMs in equal contiguous ranges, so
     // the launch is balanced whatever the row-block count; row blocks cut between CTAs are summed through scratch.
     // Without scratch, or when the vector epilogue does not apply, ranges are whole row blocks.
-    const int n_rb = (n_pairs + 63) / 64, nkb = a.in / TC_BK, total = n_rb * nkb;
+    const int n_rb = (n_pairs + 63) / 64, nkb = a.in / (Q8 ? TQ_K : TC_BK), total = n_rb * nkb;
     int units = (total + sms - 1) / sms;
-    if (units < 8) units = 8;  // at least 8 K blocks (128 KB of weights) per CTA
+    if (units < (Q8 ? 2 : 8)) units = Q8 ? 2 : 8;  // at least 8 K blocks (128 KB of weights, Q8_0: 68 KB) per CTA
     // a row block is shared by at most 6 CTAs: the merge loads 6 segments at once, beyond that it walks them one
     // round trip at a time (a [1280 x 8192] projection cut 15 ways took 41 us for 21 MB)
     if (units < (nkb + 4) / 5) units = (nkb + 4) / 5;
@@ -732,7 +903,7 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
         max_seg = 1;
     }
     dim3 grid((total + units - 1) / units);
-    LCU_CHECK_CUDA(launch_kernel(kernel, grid, dim3(TC_THREADS), smem, s, pdl, a, mw, mx, n_pairs, N, stages, units, max_seg, vec,
+    LCU_CHECK_CUDA(launch_kernel(kernel, grid, dim3(Q8 ? TQ_THREADS : TC_THREADS), smem, s, pdl, a, mw, ms, mx, n_pairs, N, stages, units, max_seg, vec,
                                  idesc, g_tc_ws, g_tc_tickets, status));
     g_linear_last_ctas = (int)grid.x;
     return LCU_OK;
@@ -748,15 +919,20 @@ int gemm_tc_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool dry
     LCU_REQUIRE(!a.tiles || (a.out % 8 == 0 && (a.tile_rows == 64 || a.tile_rows == 128 || a.tile_rows == 256) && a.n_tiles <= 65535),
                 "gemm_tc: groups of %d rows in %d tiles of %d", a.out, a.n_tiles, a.tile_rows);
     if (a.epilogue == EPI_SWIGLU) LCU_REQUIRE(a.out == 2 * a.di, "gemm_tc: swiglu needs out == 2*di");
-    if (dt == LCU_F16) return tc_launch_t<__half>(a, dt, s, pdl, dry);
-    if (dt == LCU_BF16) return tc_launch_t<__nv_bfloat16>(a, dt, s, pdl, dry);
+    if (a.w_q8) {
+        LCU_REQUIRE(dt == LCU_F16 && !a.tiles && a.epilogue <= EPI_SWIGLU, "gemm_tc: Q8_0 weights need f16 activations and a LLaMA epilogue");
+        LCU_REQUIRE(dry || ((uintptr_t)a.w_scales % 16) == 0, "gemm_tc: operands must be 16-byte aligned");
+        return tc_launch_t<__half, true>(a, dt, s, pdl, dry);
+    }
+    if (dt == LCU_F16) return tc_launch_t<__half, false>(a, dt, s, pdl, dry);
+    if (dt == LCU_BF16) return tc_launch_t<__nv_bfloat16, false>(a, dt, s, pdl, dry);
     set_error("gemm_tc: activation dtype %d unsupported", dt);
     return LCU_ERR_INVALID;
 }
 
-int gemm_tc_warm(int dt) {
+int gemm_tc_warm(int dt, bool q8) {
     GemvArgs a{};
-    a.in = 256; a.out = 256; a.n_tok = 16; a.stride_x = 256; a.epilogue = EPI_STORE;
+    a.w_q8 = q8; a.in = 256; a.out = 256; a.n_tok = 16; a.stride_x = 256; a.epilogue = EPI_STORE;
     return gemm_tc_launch(a, dt, nullptr, false, true);
 }
 

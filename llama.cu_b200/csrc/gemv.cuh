@@ -242,7 +242,7 @@ void gemm_skinny_set_scratch(void *ws, size_t ws_bytes, unsigned *tickets, int n
 constexpr int GEMM_TC_MAX_TOKENS = 65536;  // blocks of 256 on grid.y
 bool gemm_tc_supported(int in, int w_q8);
 int gemm_tc_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool dry = false);
-int gemm_tc_warm(int dt);
+int gemm_tc_warm(int dt, bool q8 = false);
 void gemm_tc_set_scratch(void *ws, size_t ws_bytes, unsigned *tickets, int n_tickets, uint32_t *status);
 // CTAs of the calling thread's most recent linear-layer launch (GEMV or batched): the peer all-reduce
 // counts one arrival per producing CTA.

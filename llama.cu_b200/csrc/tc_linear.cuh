@@ -7,7 +7,55 @@ namespace lcu {
 
 constexpr int TC_BK = 64;  // K elements per stage (128 bytes: one swizzle row)
 
+// ---- Q8_0 weights as pairs of f16: scale * q = hi + lo, hi the rounded product, lo the rest.  Exact: the product is a whole multiple
+// of 2^-24 with at most 19 bits, so both halves are f16 numbers (subnormal ones among them) wherever hi does not overflow, and f16
+// products summed in f32 lose no more than integer products scaled block by block.  Twice the MMAs of f16 weights.
+constexpr int TQ_K = 256;  // K elements per unit of the form with weights on lanes: 16 bytes of scales a row
+
 #ifdef __CUDACC__
+__device__ __forceinline__ void tc_q8_split(const uint4 &q, __half2 s, uint32_t hi[8], uint32_t lo[8]) {
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t h[2];
+        q8x4_to_h2(w[i], h[0], h[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const __half2 v = *reinterpret_cast<__half2 *>(&h[k]), p = __hmul2(v, s), r = __hfma2(v, s, __hneg2(p));
+            hi[2 * i + k] = *reinterpret_cast<const uint32_t *>(&p);
+            lo[2 * i + k] = *reinterpret_cast<const uint32_t *>(&r);
+        }
+    }
+}
+// The product of a row with a token, block by block in f32: what an output becomes whose sum is not finite (a scale times 127 beyond
+// the range of f16, or activations that are not finite themselves).
+static __device__ __noinline__ float tc_q8_row(const int8_t *q, const __half *s, const __half *x, int in) {
+    float acc = 0.f;
+    for (int b = 0; b < in / 32; ++b) {
+        float d = 0.f;
+        for (int i = 0; i < 32; ++i) d = fmaf((float)q[32 * b + i], __half2float(x[32 * b + i]), d);
+        acc = fmaf(__half2float(s[b]), d, acc);
+    }
+    return acc;
+}
+__device__ __forceinline__ float tc_q8_dot(const GemvArgs &a, int n, int row) {
+    return tc_q8_row(reinterpret_cast<const int8_t *>(a.w) + (size_t)row * a.in, reinterpret_cast<const __half *>(a.w_scales) + (size_t)row * (a.in / 32),
+                     reinterpret_cast<const __half *>(a.x) + (size_t)n * a.stride_x, a.in);
+}
+__device__ __forceinline__ void tc_q8_mend(const GemvArgs &a, int n, int row, float v[8]) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ok = ok && fabsf(v[i]) < INFINITY;
+    if (ok) return;
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i) {
+        const float r = tc_q8_dot(a, n, row + i);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)  // (no local array: every index is known)
+            if (k == i) v[k] = r;
+    }
+}
+
 // Vector form of the fused epilogues for one token and 8 consecutive outputs.  Everything a thread reads
 // from global memory for its items (residual, rotation table, page number) is fetched by tc_prefetch
 // before tc_finish stores anything: outputs may alias inputs (the residual is updated in place), so the
@@ -137,6 +185,23 @@ inline int tc_make_map(CUtensorMap *m, const void *base, int dt, uint64_t rows, 
     return LCU_OK;
 }
 
+// Q8_0: the bytes in boxes of 128 columns x 64 rows (128-byte swizzle), the scales in boxes of 8 columns x 64 rows
+inline int tc_make_q8_maps(CUtensorMap *mq, CUtensorMap *ms, const void *q, const void *scales, uint64_t rows, uint64_t cols) {
+    TcEncodeFn fn = tc_encode_fn();
+    LCU_REQUIRE(fn, "gemm_tc: cuTensorMapEncodeTiled is not available");
+    const cuuint64_t qd[2] = {cols, rows}, qs[1] = {cols}, sd[2] = {cols / 32, rows}, ss[1] = {cols / 16};
+    const cuuint32_t qb[2] = {128, 64}, sb[2] = {TQ_K / 32, 64}, es[2] = {1, 1};
+    const CUresult r1 = fn(mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(q), qd, qs, qb, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r2 = fn(ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(scales), sd, ss, sb, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS) {
+        set_error("gemm_tc: cuTensorMapEncodeTiled failed with %d, %d (Q8_0, %llu x %llu)", (int)r1, (int)r2, (unsigned long long)rows, (unsigned long long)cols);
+        return LCU_ERR_CUDA;
+    }
+    return LCU_OK;
+}
+
 inline bool tc_vec(const GemvArgs &a) {  // whether the 16-byte epilogues apply
     const bool f32 = a.epilogue == EPI_STORE_F32 || a.epilogue == EPI_CAP_F32;
     bool ok = a.stride_y % (f32 ? 4 : 8) == 0 && ((uintptr_t)a.y % 16) == 0 && (a.epilogue == EPI_SWIGLU ? a.di % 8 == 0 : a.out % 8 == 0);
@@ -150,6 +215,6 @@ inline bool tc_vec(const GemvArgs &a) {  // whether the 16-byte epilogues apply
 // 256 x up to 256 tiles on pairs of SMs for rounds of many tokens (gemm_pair.cu); the arguments are those of gemm_tc_launch.
 bool gemm_pair_takes(const GemvArgs &a);
 int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status);
-int gemm_pair_warm(int dt);
+int gemm_pair_warm(int dt, bool q8);
 
 }  // namespace lcu
