@@ -81,25 +81,35 @@ static DescLayout desc_layout(int n_tok, int n_req, int n_out, int pt_stride) {
     return L;
 }
 
+// Tiles of 64 positions that the plan below allows for: the longest context of the round, up to the next power of two, so that a
+// captured round stays valid while contexts grow within it.
+static int attn_tiles(const lcu_ctx *c, uint32_t longest) {
+    const int most = (c->desc.nctx + 63) / 64;
+    int tiles = 1;
+    while (tiles < most && (uint32_t)tiles * 64 < longest) tiles *= 2;
+    return tiles < most ? tiles : most;
+}
+
 // Split-KV plan of the attention launch for a round of n_tok tokens (flash-decoding): every CTA walks
-// `tps` 64-position tiles, the grid is deep enough for the longest context the cache allows, and a token
-// with a shorter context simply uses fewer of its CTAs.  Fixed per round shape so that a captured graph
-// stays valid as contexts grow.  Rounds with enough tokens to fill the GPU on their own (prefill) are
-// not split.
+// `tps` 64-position tiles, the grid is deep enough for `max_tiles`, and a token with a shorter context
+// simply uses fewer of its CTAs.  Planned for the round's own contexts, not for the longest that the cache allows, which cut 16
+// sequences of 100 to 290 tokens by four tiles and sent one sequence of 129 through scratch instead of a cluster (8B shape, per
+// round: 3.88 -> 3.71 ms in Q8_0, 2.81 -> 2.73 ms in f16; one sequence of 200 tokens of the 1B shape 657 -> 623 us).
+// Rounds with enough tokens to fill the GPU on their own (prefill) are not split.
 // Fewest tokens in a round for which the linear layers run as batched tensor-core kernels instead of
 // the register-blocked GEMV (measured on the 8B shapes: the GEMV wins up to 2 tokens).
 static int batched_min_tokens() { return 3; }
 
-static void attn_plan(const lcu_ctx *c, int n_tok, int *n_splits, int *tps) {
+static void attn_plan(const lcu_ctx *c, int n_tok, int max_tiles, int *n_splits, int *tps) {
     const int ctas = c->nkvh_l * n_tok;
-    const int max_tiles = (c->desc.nctx + 63) / 64;
     if (ctas >= 8 * sm_count() || max_tiles <= 1) {
         *n_splits = 1;
         *tps = max_tiles;
         return;
     }
-    // tiles per CTA: enough CTAs to fill the GPU about four times over when every context is full, at most 4
-    int t = (int)(((long)ctas * max_tiles + 4L * sm_count() - 1) / (4L * sm_count()));
+    // tiles per CTA: enough CTAs to fill the GPU about eight times over when every context is full, at most 4 (four times: 16
+    // sequences of 100 to 290 tokens of the 8B shape 3.76 instead of 3.71 ms per round)
+    int t = (int)(((long)ctas * max_tiles + 8L * sm_count() - 1) / (8L * sm_count()));
     if (t > 4) t = 4;
     if (t < 1) t = 1;
     // a round of a few tokens merges its splits inside one thread-block cluster (at most 8 CTAs): take 2 tiles per
@@ -117,10 +127,15 @@ static void attn_plan(const lcu_ctx *c, int n_tok, int *n_splits, int *tps) {
     *tps = t;
 }
 
-static int attn_splits(const lcu_ctx *c, int n_tok) {
-    int z, t;
-    attn_plan(c, n_tok, &z, &t);
-    return z;
+static int attn_splits(const lcu_ctx *c, int n_tok) {  // the deepest of every length of contexts
+    int most = 1;
+    const int tiles = attn_tiles(c, (uint32_t)c->desc.nctx);
+    for (int m = 1; ; m = m * 2 < tiles ? m * 2 : tiles) {
+        int z, t;
+        attn_plan(c, n_tok, m < tiles ? m : tiles, &z, &t);
+        if (z > most) most = z;
+        if (m >= tiles) return most;
+    }
 }
 
 // Rows of the LM head one rank holds when the head is sharded by vocabulary (0: the shape does not allow it).
@@ -711,7 +726,7 @@ int enqueue_round(lcu_ctx *c, const Round &r, lcu_kv_pair *out_dev, cudaStream_t
     };
 
     int n_splits, attn_tps;
-    attn_plan(c, r.n_tok, &n_splits, &attn_tps);
+    attn_plan(c, r.n_tok, r.attn_tiles, &n_splits, &attn_tps);
     const bool batched = c->batched_ok && r.n_tok >= batched_min_tokens();
     // GEMV rounds: the three GEMV -> GEMV edges (the edges around attention lose there); batched rounds: also attention -> O
     const int pdl_edges = pdl_edges_env >= 0 ? pdl_edges_env : (batched ? 30 : 28);
@@ -1100,6 +1115,7 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
     Round r;
     r.n_tok = n_tok; r.n_req = n_req; r.n_fast = n_fast; r.any_sampling = any_sampling; r.decode_only = decode_only;
     r.n_groups = 0;
+    r.attn_tiles = attn_tiles(c, longest);
     r.n_out = rows ? n_rows : n_req;
     r.logits_f32 = logits_dev;
     r.L = desc_layout(n_tok, n_req, r.n_out, c->pt_stride);
@@ -1193,10 +1209,10 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
         return finish(rc);
     }
     std::vector<int> key = {n_req, n_tok, n_fast, any_sampling ? 1 : 0, (int)((uintptr_t)out_dev & 0x7fffffff),
-                            (int)((uintptr_t)out_dev >> 31), c->head_shard ? 1 : 0};
+                            (int)((uintptr_t)out_dev >> 31), c->head_shard ? 1 : 0, c->stack ? 0 : r.attn_tiles};
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
-        // A captured round is keyed by its shape AND by the output buffer (a host that rotates output buffers, as the
+        // A captured round is keyed by its shape, the reach of its attention AND by the output buffer (a host that rotates output buffers, as the
         // reference's triple-buffered loop does, holds one graph per buffer): keep the table bounded
         if (c->graphs.size() >= 96) drop_graphs(c);
         cudaGraph_t graph = nullptr;
