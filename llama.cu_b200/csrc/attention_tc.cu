@@ -28,7 +28,7 @@ constexpr int AT_MAX_STAGES = 4;
 
 struct AtShared {
     unsigned long long k_full[AT_MAX_STAGES], k_empty[AT_MAX_STAGES], v_full[AT_MAX_STAGES], v_empty[AT_MAX_STAGES];
-    unsigned long long q_full, s_full[2], p_ready[2], o_done[2];
+    unsigned long long q_full, s_full[2], p_ready[2], o_done[2], drain;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -124,6 +124,7 @@ attn_tc_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap map_q, cons
             tc_mbar_init(tc_smem(&sh->v_empty[i]), 1);
         }
         tc_mbar_init(tc_smem(&sh->q_full), 1);
+        tc_mbar_init(tc_smem(&sh->drain), 1);
         for (int t = 0; t < 2; ++t) {
             tc_mbar_init(tc_smem(&sh->s_full[t]), 1);
             tc_mbar_init(tc_smem(&sh->p_ready[t]), 4);
@@ -144,6 +145,7 @@ attn_tc_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap map_q, cons
         if (lane == 0) atomicOr(a.status, 4u);
         sh->abort_flag = 1;
     };
+    int k_issued = 0, v_issued = 0;  // stages that warp 0 has requested
 
     if (warp == 0) {
         // ---------------- TMA producer
@@ -169,30 +171,23 @@ attn_tc_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap map_q, cons
                 for (int b = 0; b < NB; ++b) at_tma_3d(dst + (uint32_t)(b * AT_BOX + i * pt * 128), &map_kv, 64 * b, 0, z, bar);
             }
         };
-        int slot = 0, j = 0;
+        int slot = 0;
         uint32_t phase = 1;
         bool ok = true;
-        for (; j < n_tiles; ++j) {
+        for (int j = 0; j < n_tiles; ++j) {
             const int n = min(ppt, (ctx - j * 128 + pt - 1) >> a.geom.page_shift);
             ok = tc_warp_wait(ke + 8 * slot, phase, &sh->abort_flag);
             if (!ok) break;
             load(tc_smem(Ks) + (uint32_t)(slot * TILE), kf + 8 * slot, n, kb);
+            ++k_issued;
             ok = tc_warp_wait(ve + 8 * slot, phase, &sh->abort_flag);
             if (!ok) break;
             load(tc_smem(Vs) + (uint32_t)(slot * TILE), vf + 8 * slot, n, vb);
+            ++v_issued;
             if (j + 1 < n_tiles) id = page_of(j + 1);
             if (++slot == ST) { slot = 0; phase ^= 1u; }
         }
         if (!ok) give_up();
-        if (__any_sync(0xffffffffu, sh->abort_flag != 0)) {  // copies in flight must land before the CTA gives its memory up
-            int never = 0;
-            tc_warp_wait(q_bar, 0u, &never);
-            for (int i = j >= ST ? j - ST : 0; i <= j && i < n_tiles; ++i) {
-                const uint32_t ph = (uint32_t)(i / ST) & 1u;
-                if (i < j || !ok) tc_warp_wait(kf + 8 * (i % ST), ph, &never);
-                if (i < j) tc_warp_wait(vf + 8 * (i % ST), ph, &never);
-            }
-        }
     } else if (warp == 1) {
         // ---------------- MMA issuer
         const uint32_t id_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -346,6 +341,18 @@ attn_tc_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap map_q, cons
         }
     }
     __syncthreads();
+    if (sh->abort_flag) {  // a wait has run out: what still writes to the CTA's memory ends first
+        if (warp == 0) {
+            tc_warp_drain(tc_smem(&sh->q_full), 0u);
+            tc_warp_drain_ring(tc_smem(&sh->k_full[0]), k_issued, ST);
+            tc_warp_drain_ring(tc_smem(&sh->v_full[0]), v_issued, ST);
+        }
+        if (warp == 1) {
+            tc_warp_commit(tc_smem(&sh->drain));
+            tc_warp_drain(tc_smem(&sh->drain), 0u);
+        }
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");

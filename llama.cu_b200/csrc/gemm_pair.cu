@@ -12,7 +12,8 @@
 // Measured (products alone, weights beyond L2): 28672 x 4096 with 997 tokens 356 -> 195 us (1.20 PFLOP/s), with 8000 tokens 2543 ->
 // 1356 us (1.39 PFLOP/s; cuBLAS 1267 us), 4096 x 14336 with 997 tokens 115 -> 104 us, against one CTA per 128 x 256 tile.
 // Barriers `full` and `tmem_empty` count in the even CTA; `empty` and `tmem_full` are signalled in both by tcgen05.commit.
-// Every mbarrier wait is bounded as in gemm_tc.cu: on expiry a status bit is set and the remaining work is skipped.
+// Every mbarrier wait is bounded as in gemm_tc.cu: on expiry a status bit is set and the remaining work is skipped; the pair leaves
+// when its copies have landed and its MMAs have ended.
 #include <map>
 #include <mutex>
 
@@ -40,7 +41,7 @@ constexpr int TPQ_Q_BYTES = TPQ_ROWS * TQ_K, TPQ_G_BYTES = TPQ_Q_BYTES + TPQ_ROW
 constexpr int TP_COLS = 256;                     // TMEM columns of one accumulator
 
 struct TpShared {
-    unsigned long long full[TP_STAGES], empty[TP_STAGES], tmem_full[2], tmem_empty[2], g_full[TPQ_GROUPS], g_empty[TPQ_GROUPS];
+    unsigned long long full[TP_STAGES], empty[TP_STAGES], tmem_full[2], tmem_empty[2], g_full[TPQ_GROUPS], g_empty[TPQ_GROUPS], drain;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -117,6 +118,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
             tc_mbar_init(tc_smem(&sh->g_full[i]), 1);
             tc_mbar_init(tc_smem(&sh->g_empty[i]), 8);
         }
+        tc_mbar_init(tc_smem(&sh->drain), 1);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -129,6 +131,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
     tp_cluster_sync();  // the peer's barriers exist
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh->tmem_base;
+    int issued = 0;  // stages (warp 0) and groups (the last warp of the Q8_0 form) that this warp has requested
 
     if (warp == 0) {
         // ---------------- TMA producer of this CTA's operands; their bytes count on the even CTA's barrier.  Places in the ring,
@@ -156,7 +159,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 for (int j = 0; j < early; ++j) weights(j, j * TC_BK, nt);
                 grid_dep_wait();
                 for (int j = 0; j < early; ++j) acts(j, j * TC_BK, mt);
-                kb = early;
+                kb = issued = early;
                 slot = early == STAGES ? 0 : early;
                 phase = early == STAGES ? 0 : 1;
                 primed = true;
@@ -170,6 +173,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 }
                 weights(slot, kb * TC_BK, nt);
                 acts(slot, kb * TC_BK, mt);
+                ++issued;
                 if (++slot == STAGES) { slot = 0; phase ^= 1u; }
             }
         }
@@ -207,7 +211,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                     tp_commit_both(empty0 + 8 * slot);
                     if (++slot == STAGES) { slot = 0; phase ^= 1u; }
                 }
-                tp_commit_both(tc_smem(&sh->tmem_full[ab]));
+                if (!stop) tp_commit_both(tc_smem(&sh->tmem_full[ab]));  // (an accumulator that lacks K blocks is never handed over)
             }
         }
     } else if (Q8 && warp == TPQ_THREADS / 32 - 1) {
@@ -229,6 +233,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 tc_warp_tma_2d(dst, &map_w, kb * TC_BK, row, bar);
                 tc_warp_tma_2d(dst + TPQ_Q_BYTES / 2, &map_w, kb * TC_BK + 128, row, bar);
                 tc_warp_tma_2d(dst + TPQ_Q_BYTES, &map_s, kb * 2, row, bar);
+                ++issued;
                 if (++slot == TPQ_GROUPS) { slot = 0; phase ^= 1u; }
             }
         }
@@ -355,8 +360,8 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
         for (int tile = pair; tile < n_tiles; tile += n_pairs, ++ti) {
             const int mt = tile % n_mt, nt = tile / n_mt;
             const int ab = ti & 1;
-            if (!tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag)) {
-                atomicOr(status, 4u);
+            if (!__all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag))) {  // (the loads take the whole warp)
+                if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
                 break;
             }
@@ -410,6 +415,15 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
     // ---------------- tail: both CTAs are done with each other's barriers and accumulators
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (sh->abort_flag) {
+        // both CTAs' operands count on the even CTA's barriers, and its MMAs read both CTAs' memory: it waits for both
+        if (rank == 0 && warp == 0) tc_warp_drain_ring(tc_smem(&sh->full[0]), issued, STAGES);
+        if (rank == 0 && warp == 1) {
+            tp_commit_both(tc_smem(&sh->drain));
+            tc_warp_drain(tc_smem(&sh->drain), 0u);
+        }
+        if (Q8 && warp == TPQ_THREADS / 32 - 1) tc_warp_drain_ring(tc_smem(&sh->g_full[0]), issued, TPQ_GROUPS);
+    }
     tp_cluster_sync();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

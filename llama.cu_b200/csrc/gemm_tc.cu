@@ -17,7 +17,7 @@
 //   - matrices with few rows are split along K across CTAs (grid.y); partial sums go through
 //     scratch memory and the last CTA of a row block to arrive adds them in split order.
 // Every mbarrier wait is bounded by a wall-clock limit: on expiry the kernel records a status bit,
-// skips the remaining work, frees its TMEM and returns.
+// skips the remaining work, waits for its own copies and MMAs, frees its TMEM and returns.
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -54,11 +54,22 @@ __device__ __forceinline__ void tq_st16(uint32_t taddr, const uint32_t *r) {
 }
 
 struct TcShared {
-    unsigned long long full[TC_MAX_STAGES], empty[TC_MAX_STAGES], tmem_full[2], tmem_empty[2], a_full[TQ_RING], a_empty[TQ_RING];
+    unsigned long long full[TC_MAX_STAGES], empty[TC_MAX_STAGES], tmem_full[2], tmem_empty[2], a_full[TQ_RING], a_empty[TQ_RING], drain;
     uint32_t tmem_base;
     int abort_flag;
     int last;
 };
+
+// Behind the CTA's last barrier: where a wait has run out, what still writes to its memory ends first.
+__device__ __forceinline__ void tc_leave(TcShared *sh, int warp, int issued, int n_stages) {
+    if (!sh->abort_flag) return;
+    if (warp == 0) tc_warp_drain_ring(tc_smem(&sh->full[0]), issued, n_stages);
+    if (warp == 1) {
+        tc_warp_commit(tc_smem(&sh->drain));
+        tc_warp_drain(tc_smem(&sh->drain), 0u);
+    }
+    __syncthreads();
+}
 
 // Persistent: grid = min(tiles, SMs); a tile is (row block of 128 rows = 64 pairs, K split); CTA c takes
 // tiles c, c + grid, ...  The shared-memory ring keeps running across tiles and the accumulator is
@@ -106,6 +117,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             tc_mbar_init(tc_smem(&sh->a_full[i]), 4);
             tc_mbar_init(tc_smem(&sh->a_empty[i]), 1);
         }
+        tc_mbar_init(tc_smem(&sh->drain), 1);
         sh->abort_flag = 0;
         sh->last = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -118,6 +130,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh->tmem_base;
+    int issued = 0;  // stages that warp 0 has requested
 
     if (warp == 0) {
         // ---------------- TMA producer: units u_begin .. u_end - 1, unit = (row block, K block).  The whole warp runs the loop (one
@@ -160,6 +173,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             acts(j, kb_x);
             if (++kb_x == nkb) kb_x = 0;
         }
+        issued = first;
         uint32_t phase = 0;
         for (int j = first, slot = 0; j < n_units; ++j) {  // (only a full ring leaves units over)
             if (!tc_warp_wait(empty0 + 8 * slot, phase, &sh->abort_flag)) {
@@ -169,6 +183,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             }
             weights(slot, kb, rb);
             acts(slot, kb);
+            ++issued;
             if (++kb == nkb) { kb = 0; ++rb; }
             if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
@@ -226,6 +241,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                 tc_warp_commit(empty0 + 8 * slot);  // the stage is free once these MMAs have read it
                 if (++slot == n_stages) { slot = 0; phase ^= 1u; }
             }
+            if (sh->abort_flag) break;                       // (one that lacks K blocks is never handed over)
             tc_warp_commit(tc_smem(&sh->tmem_full[ab]));     // accumulator complete
             u += kb1 - kb0;
             kb0 = Q8 && kb1 < nkb ? kb1 : 0;
@@ -323,10 +339,10 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                     if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&sh->tmem_empty[ub])) : "memory");
                 }
             } else {
-                ok = tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag);
+                ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag));  // (the loads take the whole warp)
             }
             if (!ok) {
-                atomicOr(status, 4u);
+                if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -503,6 +519,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     p2p_signal(a.push);  // no-op without tensor parallelism
     __syncthreads();
+    tc_leave(sh, warp, issued, n_stages);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tm_cols) : "memory");
@@ -573,6 +590,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
             tc_mbar_init(tc_smem(&sh->empty[i]), 1);
         }
         tc_mbar_init(tc_smem(&sh->tmem_full[0]), 1);
+        tc_mbar_init(tc_smem(&sh->drain), 1);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -586,6 +604,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
     const uint32_t tmem = sh->tmem_base;
 
     bool ok = true;  // epilogue warps: the accumulator is complete
+    int issued = 0;  // stages that warp 0 has requested
     if (warp == 0) {
         // ---------------- TMA producer (weights of the first ring before the dependency wait, whole warp: as in gemm_tc_kernel)
         const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]), smem0 = tc_smem(smem);
@@ -603,6 +622,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
         for (int j = 0; j < first; ++j) weights(j, (kb0 + j) * TC_BK);
         grid_dep_wait();
         for (int j = 0; j < first; ++j) acts(j, (kb0 + j) * TC_BK);
+        issued = first;
         uint32_t phase = 0;
         for (int kb = kb0 + first, slot = 0; kb < kb1; ++kb) {
             if (!tc_warp_wait(empty0 + 8 * slot, phase, &sh->abort_flag)) {
@@ -612,6 +632,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
             }
             weights(slot, kb * TC_BK);
             acts(slot, kb * TC_BK);
+            ++issued;
             if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
     } else if (warp == 1) {
@@ -631,11 +652,11 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
             tc_warp_commit(empty0 + 8 * slot);
             if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
-        tc_warp_commit(tc_smem(&sh->tmem_full[0]));
+        if (!sh->abort_flag) tc_warp_commit(tc_smem(&sh->tmem_full[0]));  // (an accumulator that lacks K blocks is never handed over)
     } else if (warp >= 2) {
-        ok = tc_mbar_wait(tc_smem(&sh->tmem_full[0]), 0u, &sh->abort_flag);
+        ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[0]), 0u, &sh->abort_flag));  // (the loads take the whole warp)
         if (!ok) {
-            atomicOr(status, 4u);
+            if (lane == 0) atomicOr(status, 4u);
             sh->abort_flag = 1;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -702,6 +723,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
     }
     p2p_signal(a.push);  // no-op without tensor parallelism
     __syncthreads();
+    tc_leave(sh, warp, issued, n_stages);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tm_cols) : "memory");

@@ -291,7 +291,7 @@ latent_tc_kernel(const LatentAttnArgs a, const __grid_constant__ CUtensorMap map
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 lt_arrive(tc_smem(&sh->z_ready));
             }
-            ok = ok && tc_mbar_wait(tc_smem(&sh->s_full), (uint32_t)(tile - tile0) & 1u, &sh->abort_flag);
+            ok = __all_sync(0xffffffffu, ok && tc_mbar_wait(tc_smem(&sh->s_full), (uint32_t)(tile - tile0) & 1u, &sh->abort_flag));  // (the loads take the whole warp)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t raw[N];
             if (ok) {

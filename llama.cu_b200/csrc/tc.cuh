@@ -36,6 +36,18 @@ __device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, vola
         if ((it & 255u) == 0 && (*abort_flag || tc_ns() - t0 > TC_WAIT_NS)) return false;
     }
 }
+// ---- After a wait has run out a CTA may leave only when nothing writes to its memory any more: its copies have landed and its MMAs
+// have ended.  A barrier that stays open (an arrival that never came) ends by a limit far above what a copy takes.
+constexpr unsigned long long TC_DRAIN_NS = 10000000ull;
+__device__ __forceinline__ void tc_warp_drain(uint32_t bar, uint32_t parity) {
+    const unsigned long long t0 = tc_ns();
+    while (!__all_sync(0xffffffffu, tc_mbar_try(bar, parity)) && __all_sync(0xffffffffu, tc_ns() - t0 < TC_DRAIN_NS)) {
+    }
+}
+// a ring of `stages` barriers that was filled `issued` times: only the last fill of a stage can be open
+__device__ __forceinline__ void tc_warp_drain_ring(uint32_t full0, int issued, int stages) {
+    for (int f = issued > stages ? issued - stages : 0; f < issued; ++f) tc_warp_drain(full0 + 8 * (f % stages), (uint32_t)(f / stages) & 1u);
+}
 // ---- forms for a whole converged warp: one elected lane issues, and nothing but the instruction depends on the lane, so the
 // compiler keeps operands and loop in uniform registers (issued from a `lane == 0` branch, four MMAs take 270 cycles to issue)
 __device__ __forceinline__ bool tc_warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
