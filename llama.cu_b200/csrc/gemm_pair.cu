@@ -290,7 +290,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
         if constexpr (Q8) {
             const int q = warp & 3, h = (warp - 2) >> 2;
             const int c_a = swiglu ? h * 32 : h * 64, c_b = swiglu ? TPQ_ROWS + h * 32 : c_a + 32;
-            int ti = 0;
+            int ti = 0, known = TQ_UNKNOWN, known_n = -1;
             bool ok = true;
             grid_dep_wait();
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
@@ -319,6 +319,9 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                         asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
                 }
                 if (!ok) break;
+                const int r0 = nt * step + c_a;
+                if (n != known_n) { known = TQ_UNKNOWN; known_n = n; }
+                tc_q8_mend<64>(a, n < a.n_tok, n, r0, swiglu ? a.di : a.out, swiglu ? a.di + r0 : r0 + 32, sum, known);
                 if (n >= a.n_tok) continue;
                 if (swiglu) {
 #pragma unroll
@@ -326,8 +329,6 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                         const int first = nt * step + c_a + c;
                         if (first + 8 > a.di) continue;
                         TcPre pre;
-                        tc_q8_mend(a, n, first, sum + c);
-                        tc_q8_mend(a, n, a.di + first, sum + 32 + c);
                         tc_finish<T>(a, n, first, sum + c, sum + 32 + c, pre);
                     }
                 } else {
@@ -341,7 +342,6 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
                             if (first + 8 * k + 8 > a.out) continue;
-                            tc_q8_mend(a, n, first + 8 * k, sum + c + 8 * k);
                             tc_finish<T>(a, n, first + 8 * k, sum + c + 8 * k, sum + c + 8 * k, pre[k]);
                         }
                     }

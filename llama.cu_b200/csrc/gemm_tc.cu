@@ -58,6 +58,7 @@ struct TcShared {
     uint32_t tmem_base;
     int abort_flag;
     int last;
+    int known[64];  // Q8_0: what the tokens' activations hold (tc_q8_mend)
 };
 
 // Behind the CTA's last barrier: where a wait has run out, what still writes to its memory ends first.
@@ -118,6 +119,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             tc_mbar_init(tc_smem(&sh->a_empty[i]), 1);
         }
         tc_mbar_init(tc_smem(&sh->drain), 1);
+        for (int i = 0; Q8 && i < 64; ++i) sh->known[i] = TQ_UNKNOWN;
         sh->abort_flag = 0;
         sh->last = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -384,31 +386,38 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                 for (int idx = et; idx < chunks * N; idx += 128, ++cnt) {
                     int c = idx % chunks, n = idx / chunks;
                     int first = swiglu ? rb * 64 + 8 * c : rb * TC_BM + 8 * c;
-                    if (!(n < a.n_tok && first + 8 <= (swiglu ? a.di : a.out))) continue;
-                    float v[8], u[8];
+                    const bool mine = n < a.n_tok && first + 8 <= (swiglu ? a.di : a.out);
+                    if (!Q8 && !mine) continue;
+                    float v[16];  // 8 outputs (SwiGLU: their gates, then their ups)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         v[i] = stg[(8 * c + i) * (N + 1) + n];
-                        u[i] = swiglu ? stg[(64 + 8 * c + i) * (N + 1) + n] : 0.f;
+                        v[8 + i] = swiglu ? stg[(64 + 8 * c + i) * (N + 1) + n] : 0.f;
                     }
-                    if constexpr (Q8) {
-                        tc_q8_mend(a, n, first, v);
-                        if (swiglu) tc_q8_mend(a, n, a.di + first, u);
+                    if constexpr (Q8) {  // (16 * N and 8 * N items: the threads go round together)
+                        int known = sh->known[n];
+                        if (swiglu) tc_q8_mend<16>(a, mine, n, first, a.di, a.di + first, v, known);
+                        else tc_q8_mend<8>(a, mine, n, first, a.out, first + 4, v, known);
+                        if (!mine) continue;
+                        if (known) sh->known[n] = known;
                     }
-                    tc_finish<T>(a, n, first, v, u, pre[cnt]);
+                    tc_finish<T>(a, n, first, v, v + 8, pre[cnt]);
                 }
             } else if (whole) {
                 for (int idx = et; idx < items; idx += 128) {
                     int j = idx / N, n = idx - j * N;
                     int p = rb * 64 + j;
-                    if (p >= n_pairs || n >= a.n_tok) continue;
+                    const bool mine = p < n_pairs && n < a.n_tok;
+                    if (!Q8 && !mine) continue;
                     int ra = swiglu ? j : 2 * j, rb2 = swiglu ? 64 + j : 2 * j + 1;
-                    float va = stg[ra * (N + 1) + n], vb = stg[rb2 * (N + 1) + n];
+                    float v[2] = {stg[ra * (N + 1) + n], stg[rb2 * (N + 1) + n]};
                     if constexpr (Q8) {
-                        if (!(fabsf(va) < INFINITY)) va = tc_q8_dot(a, n, swiglu ? p : 2 * p);
-                        if (!(fabsf(vb) < INFINITY)) vb = tc_q8_dot(a, n, swiglu ? a.di + p : 2 * p + 1);
+                        int known = sh->known[n];
+                        tc_q8_mend<2>(a, mine, n, swiglu ? p : 2 * p, a.out, swiglu ? a.di + p : 2 * p + 1, v, known);
+                        if (!mine) continue;
+                        if (known) sh->known[n] = known;
                     }
-                    gemv_epilogue<T>(a, p, n, va, vb);
+                    gemv_epilogue<T>(a, p, n, v[0], v[1]);
                 }
             } else {
                 // the row block is shared (the host only cuts row blocks when the vector epilogue applies).  Partial
@@ -476,16 +485,19 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                         for (int idx = et; idx < 8 * N; idx += 128) {
                             const int c = idx & 7, n = idx >> 3;
                             const int first = rb * 64 + 8 * c;
-                            if (!(n < a.n_tok && first + 8 <= a.di)) continue;
-                            float g8[8], u8[8];
-                            const float *r = tile0 + (size_t)n * TC_BM + 8 * c;
-                            merge2(r, r + 64, g8, u8);
+                            const bool mine = n < a.n_tok && first + 8 <= a.di;
+                            if (!Q8 && !mine) continue;
+                            float v[16];  // gates, ups
+                            const float *r = tile0 + (size_t)(mine ? n : 0) * TC_BM + 8 * c;
+                            merge2(r, r + 64, v, v + 8);
                             if constexpr (Q8) {
-                                tc_q8_mend(a, n, first, g8);
-                                tc_q8_mend(a, n, a.di + first, u8);
+                                int known = sh->known[n];
+                                tc_q8_mend<16>(a, mine, n, first, a.di, a.di + first, v, known);
+                                if (!mine) continue;
+                                if (known) sh->known[n] = known;
                             }
                             TcPre pre;
-                            tc_finish<T>(a, n, first, g8, u8, pre);
+                            tc_finish<T>(a, n, first, v, v + 8, pre);
                         }
                     } else {
                         // two items per pass: 8 consecutive rows of token n and of token n + 8 (idx and idx + 128)
@@ -494,17 +506,20 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                             const int first = rb * TC_BM + 8 * c;
                             const bool rows_ok = first + 8 <= a.out;
                             const bool v0 = rows_ok && n0 < a.n_tok, v1 = rows_ok && n1 < a.n_tok && idx + 128 < 16 * N;
-                            if (!v0 && !v1) continue;
+                            if (!Q8 && !v0 && !v1) continue;
                             TcPre pre0, pre1;
                             if (v0) tc_prefetch<T>(a, n0, first, pre0);
                             if (v1) tc_prefetch<T>(a, n1, first, pre1);
                             float o0[8], o1[8];
-                            const float *r0 = tile0 + (size_t)(v0 ? n0 : n1) * TC_BM + 8 * c;
-                            const float *r1 = tile0 + (size_t)(v1 ? n1 : n0) * TC_BM + 8 * c;
+                            const float *r0 = tile0 + (size_t)(v0 ? n0 : v1 ? n1 : 0) * TC_BM + 8 * c;
+                            const float *r1 = tile0 + (size_t)(v1 ? n1 : v0 ? n0 : 0) * TC_BM + 8 * c;
                             merge2(r0, r1, o0, o1);
                             if constexpr (Q8) {
-                                if (v0) tc_q8_mend(a, n0, first, o0);
-                                if (v1) tc_q8_mend(a, n1, first, o1);
+                                int k0 = sh->known[n0], k1 = sh->known[n1];
+                                tc_q8_mend<8>(a, v0, n0, first, a.out, first + 4, o0, k0);
+                                tc_q8_mend<8>(a, v1, n1, first, a.out, first + 4, o1, k1);
+                                if (v0 && k0) sh->known[n0] = k0;
+                                if (v1 && k1) sh->known[n1] = k1;
                             }
                             if (v0) tc_finish<T>(a, n0, first, o0, zero8, pre0);
                             if (v1) tc_finish<T>(a, n1, first, o1, zero8, pre1);

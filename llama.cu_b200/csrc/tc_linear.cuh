@@ -8,7 +8,7 @@ namespace lcu {
 constexpr int TC_BK = 64;  // K elements per stage (128 bytes: one swizzle row)
 
 // ---- Q8_0 weights as pairs of f16: scale * q = hi + lo, hi the rounded product, lo the rest.  Exact: the product is a whole multiple
-// of 2^-24 with at most 19 bits, so both halves are f16 numbers (subnormal ones among them) wherever hi does not overflow, and f16
+// of 2^-24 with at most 19 bits, so both halves are f16 numbers (subnormal ones among them) wherever hi does not overflow (tc_q8_mend), and f16
 // products summed in f32 lose no more than integer products scaled block by block.  Twice the MMAs of f16 weights.
 constexpr int TQ_K = 256;  // K elements per unit of the form with weights on lanes: 16 bytes of scales a row
 
@@ -27,33 +27,184 @@ __device__ __forceinline__ void tc_q8_split(const uint4 &q, __half2 s, uint32_t 
         }
     }
 }
-// The product of a row with a token, block by block in f32: what an output becomes whose sum is not finite (a scale times 127 beyond
-// the range of f16, or activations that are not finite themselves).
-static __device__ __noinline__ float tc_q8_row(const int8_t *q, const __half *s, const __half *x, int in) {
-    float acc = 0.f;
-    for (int b = 0; b < in / 32; ++b) {
-        float d = 0.f;
-        for (int i = 0; i < 32; ++i) d = fmaf((float)q[32 * b + i], __half2float(x[32 * b + i]), d);
-        acc = fmaf(__half2float(s[b]), d, acc);
-    }
-    return acc;
-}
-__device__ __forceinline__ float tc_q8_dot(const GemvArgs &a, int n, int row) {
-    return tc_q8_row(reinterpret_cast<const int8_t *>(a.w) + (size_t)row * a.in, reinterpret_cast<const __half *>(a.w_scales) + (size_t)row * (a.in / 32),
-                     reinterpret_cast<const __half *>(a.x) + (size_t)n * a.stride_x, a.in);
-}
-__device__ __forceinline__ void tc_q8_mend(const GemvArgs &a, int n, int row, float v[8]) {
-    bool ok = true;
+// Sums that are not finite: the split has overflowed (a scale times 127 beyond the range of f16), or the activations are not finite
+// themselves and an infinity has met a low half that is zero or of the other sign.  Then the products are taken block by block in
+// f32; the whole warp works on one token, for four rows per lane (below 0: none):
+//   a NaN among the activations     every product is NaN, as the sums are already;
+//   infinities                      only they and blocks whose scale is not finite decide, so a lane walks those for its own rows;
+//   finite activations              the lanes share the blocks of one row after the other.
+// A round waits for its slowest token, so this may not cost much more than the products themselves.  28672 x 4096, against one thread
+// per product: all of 500 tokens NaN 256 -> 0.24 ms (finite 0.23, mma.sync kernel 1.04), one of 64 tokens 2.3 -> 0.067 ms (finite
+// 0.064), infinities in all of 500 tokens 256 -> 1.8 to 3 ms (of one overflow, only the next matrix sees infinities: norms turn them
+// into NaN).
+enum { TQ_UNKNOWN = 0, TQ_FINITE, TQ_INF, TQ_NAN };  // what a token's activations hold
+template <int R>
+struct TqRows {
+    float v[R];
+    int known;
+};
+template <int R>
+__device__ __noinline__ TqRows<R> tc_q8_rows(const int8_t *q, const __half *s, const __half *x, int in, int4 rows, int known) {
+    const int lane = threadIdx.x & 31, nb = in / 32, row[4] = {rows.x, rows.y, rows.z, rows.w};
+    TqRows<R> o;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) ok = ok && fabsf(v[i]) < INFINITY;
-    if (ok) return;
+    for (int r = 0; r < R; ++r) o.v[r] = 0.f;
+    o.known = known;
+    auto load = [&](int k, uint4 v[8]) {  // this lane's eight of every 256 activations, 2048 at once (in % 256 == 0: lanes go round together)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = k + 256 * j < in ? *reinterpret_cast<const uint4 *>(x + k + 256 * j) : make_uint4(0, 0, 0, 0);
+    };
+    if (known == TQ_UNKNOWN) {
+        unsigned top = 0;  // the largest magnitudes, as bits
+        bool nan = false;
+        for (int k = lane * 8; k < in && !nan; k += 2048) {
+            uint4 v[8];
+            load(k, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const unsigned w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) top = __vmaxu2(top, w[i] & 0x7fff7fffu);
+            }
+            nan = __any_sync(0xffffffffu, (top & 0xffffu) > 0x7c00u || (top >> 16) > 0x7c00u);
+        }
+        o.known = nan ? TQ_NAN : __any_sync(0xffffffffu, (top & 0xffffu) == 0x7c00u || (top >> 16) == 0x7c00u) ? TQ_INF : TQ_FINITE;
+    }
+    if (o.known == TQ_NAN) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) o.v[r] = NAN;
+        return o;
+    }
+    if (o.known == TQ_INF) {
+        for (int k0 = 0; k0 < in; k0 += 2048) {
+            uint4 v[8];
+            load(k0 + lane * 8, v);
+            unsigned long long inf = 0, neg = 0;  // which of this lane's 64, and their signs
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const unsigned w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const unsigned h = w[i >> 1] >> (16 * (i & 1));
+                    inf |= (unsigned long long)((h & 0x7fffu) == 0x7c00u) << (8 * j + i);
+                    neg |= (unsigned long long)(h >> 15 & 1u) << (8 * j + i);
+                }
+            }
+            for (unsigned lanes = __ballot_sync(0xffffffffu, inf != 0); lanes; lanes &= lanes - 1) {
+                const int l = __ffs(lanes) - 1;
+                const unsigned long long sign = __shfl_sync(0xffffffffu, neg, l);
+                for (unsigned long long of = __shfl_sync(0xffffffffu, inf, l); of; of &= of - 1) {
+                    const int i = __ffsll((long long)of) - 1, k = k0 + (i >> 3) * 256 + l * 8 + (i & 7);
+                    const float xi = sign >> i & 1ull ? -INFINITY : INFINITY;
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        if (row[r] >= 0) o.v[r] = fmaf(__half2float(s[(size_t)row[r] * nb + k / 32]), (float)q[(size_t)row[r] * in + k] * xi, o.v[r]);
+                    bool open = false;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) open = open || (row[r] >= 0 && o.v[r] == o.v[r]);
+                    if (!__any_sync(0xffffffffu, open)) return o;
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (row[r] >= 0) {
+                const uint4 *sr = reinterpret_cast<const uint4 *>(s + (size_t)row[r] * nb);  // eight scales each
+                for (int c = 0; c < nb / 8; ++c) {
+                    const uint4 v = sr[c];
+                    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+                    bool odd = false;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) odd = odd || (w[i] & 0x7c00u) == 0x7c00u || (w[i] & 0x7c000000u) == 0x7c000000u;
+                    for (int b = 8 * c; odd && b < 8 * c + 8; ++b) {
+                        const float sc = __half2float(s[(size_t)row[r] * nb + b]);
+                        if (fabsf(sc) < INFINITY) continue;
+                        float d = 0.f;
+                        for (int i = 32 * b; i < 32 * b + 32; ++i) d = fmaf((float)q[(size_t)row[r] * in + i], __half2float(x[i]), d);
+                        o.v[r] = fmaf(sc, d, o.v[r]);
+                    }
+                }
+            }
+        return o;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        for (unsigned lanes = __ballot_sync(0xffffffffu, row[r] >= 0); lanes; lanes &= lanes - 1) {
+            const int l = __ffs(lanes) - 1;
+            const size_t at = (size_t)__shfl_sync(0xffffffffu, row[r], l);
+            float sum = 0.f;
+            for (int b = lane; b < nb; b += 32) {
+                float d = 0.f;
+                for (int i = 32 * b; i < 32 * b + 32; ++i) d = fmaf((float)q[at * in + i], __half2float(x[i]), d);
+                sum = fmaf(__half2float(s[at * nb + b]), d, sum);
+            }
+#pragma unroll
+            for (int k = 16; k; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+            if (lane == l) o.v[r] = sum;
+        }
+    return o;
+}
+// (apart from the kernels, whose registers the values leave only when this is called)
+template <int CNT>
+__device__ __noinline__ int tc_q8_slow(const int8_t *q, const __half *s, const __half *x, int stride_x, int in, int out, bool todo, int n, int row0, int lim0, int row1,
+                                       int known, float *v) {
+    const int lane = threadIdx.x & 31;
+    constexpr int R = CNT == 64 ? 2 : 4;
+    unsigned bad[2] = {0u, 0u};
+#pragma unroll
+    for (int i = 0; i < CNT; ++i)
+        if (!(fabsf(v[i]) < INFINITY) && (i < CNT / 2 ? row0 + i < lim0 : row1 + i - CNT / 2 < out)) bad[i / 32] |= 1u << (i & 31);
 #pragma unroll 1
-    for (int i = 0; i < 8; ++i) {
-        const float r = tc_q8_dot(a, n, row + i);
+    for (unsigned lanes = __ballot_sync(0xffffffffu, todo); lanes;) {
+        const int src = __ffs(lanes) - 1, tok = __shfl_sync(0xffffffffu, n, src);
+        const unsigned same = CNT == 64 ? 1u << src : __ballot_sync(0xffffffffu, todo && n == tok);
+        lanes &= ~same;
+        int row[4] = {-1, -1, -1, -1};
 #pragma unroll
-        for (int k = 0; k < 8; ++k)  // (no local array: every index is known)
-            if (k == i) v[k] = r;
+        for (int r = 0; r < R; ++r) {  // item 32 r + lane: value i of the m-th of these lanes
+            const int m = (32 * r + lane) / CNT, i = (32 * r + lane) % CNT, l = CNT == 64 ? src : m < __popc(same) ? (int)__fns(same, 0, m + 1) : -1, at = l < 0 ? 0 : l;
+            const unsigned b0 = __shfl_sync(0xffffffffu, bad[0], at), b1 = __shfl_sync(0xffffffffu, bad[1], at);
+            const int f0 = __shfl_sync(0xffffffffu, row0, at), f1 = __shfl_sync(0xffffffffu, row1, at);
+            row[r] = l >= 0 && ((i < 32 ? b0 : b1) >> (i & 31) & 1u) ? (i < CNT / 2 ? f0 + i : f1 + i - CNT / 2) : -1;
+        }
+        const TqRows<R> p = tc_q8_rows<R>(q, s, x + (size_t)tok * stride_x, in, make_int4(row[0], row[1], row[2], row[3]),
+                                    __shfl_sync(0xffffffffu, known, src));
+        const bool here = same >> lane & 1u;
+        if (here) known = p.known;
+        if (p.known == TQ_NAN) continue;  // (so are the sums)
+        const int first = CNT == 64 ? 0 : __popc(same & ((1u << lane) - 1u)) * CNT;
+#pragma unroll
+        for (int i = 0; i < CNT; ++i) {
+            const int w = first + i;
+            float t = 0.f;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (CNT == 64 && r != i / 32) continue;
+                const float got = __shfl_sync(0xffffffffu, p.v[r], w & 31);
+                if (CNT == 64 || r == w >> 5) t = got;
+            }
+            if (here && (bad[i / 32] >> (i & 31) & 1u)) v[i] = t;
+        }
     }
+    return known;
+}
+// Replaces the sums of token n that are not finite (`mine`: the lane has a token).  v[i]: weight row row0 + i (below lim0), from CNT / 2
+// on row1 + i - CNT / 2 (below a.out).  Lanes with the same token (no more than 128 / CNT of them; one of 64) have theirs done together.
+// `known` stays with the token.  All lanes of the warp come here.
+template <int CNT>
+__device__ __forceinline__ void tc_q8_mend(const GemvArgs &a, bool mine, int n, int row0, int lim0, int row1, float *v, int &known) {
+    float z = 0.f;
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) z = fmaf(v[i], 0.f, z);  // 0, or NaN
+    const bool todo = mine && z != 0.f && known != TQ_NAN;
+    if (!__any_sync(0xffffffffu, todo)) return;
+    float w[CNT];
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) w[i] = v[i];
+    known = tc_q8_slow<CNT>(reinterpret_cast<const int8_t *>(a.w), reinterpret_cast<const __half *>(a.w_scales), reinterpret_cast<const __half *>(a.x), a.stride_x, a.in,
+                            a.out, todo, n, row0, lim0, row1, known, w);
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) v[i] = w[i];
 }
 
 // Vector form of the fused epilogues for one token and 8 consecutive outputs.  Everything a thread reads
