@@ -321,7 +321,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 if (!ok) break;
                 const int r0 = nt * step + c_a;
                 if (n != known_n) { known = TQ_UNKNOWN; known_n = n; }
-                tc_q8_mend<64>(a, n < a.n_tok, n, r0, swiglu ? a.di : a.out, swiglu ? a.di + r0 : r0 + 32, sum, known);
+                tc_q8_mend<64>(a, n < a.n_tok, n, r0, swiglu ? a.di : a.out, swiglu ? a.di + r0 : r0 + 32, sum, &known);
                 if (n >= a.n_tok) continue;
                 if (swiglu) {
 #pragma unroll

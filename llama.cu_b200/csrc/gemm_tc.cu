@@ -1,14 +1,14 @@
 // Batched `Linear` on the 5th-generation tensor cores: tcgen05.mma with TMA-fed shared-memory
 // operands and the accumulator in tensor memory (TMEM) — for 9..64 tokens per pass (batched decode
-// rounds and prefill chunks).  Same operator as llama.cu/src/op/linear.rs:17-120 (the reference
+// rounds and prefill chunks), with Q8_0 weights from 3 tokens on.  Same operator as llama.cu/src/op/linear.rs:17-120 (the reference
 // calls cuBLAS GemmEx with m = out, n = bucketed token count, k = in).
 //
 // The GEMM is computed "swapped": D[128 weight rows x N tokens] += W_tile[128 x 64] · X[N x 64]^T,
-// so the weight dimension fills the 128-row MMA and the small token block is N (16, 32 or 64).
-//   - warp 0 (one elected lane): TMA producer — cp.async.bulk.tensor.2d loads of the weight tile (two
+// so the weight dimension fills the 128-row MMA and the small token block is N (16, 32 or 64; Q8_0 also 48).
+//   - warp 0 (as a whole; one elected lane issues): TMA producer — cp.async.bulk.tensor.2d loads of the weight tile (two
 //     64-row boxes) and of the activation tile into a ring of stages, 128-byte swizzle,
 //     completion on mbarriers.  Each weight byte is read once from HBM;
-//   - warp 1 (one elected lane): MMA issuer — four tcgen05.mma (K = 16 each) per stage, accumulating into
+//   - warp 1 (likewise): MMA issuer — four tcgen05.mma (K = 16 each) per stage, accumulating into
 //     TMEM; tcgen05.commit frees the stage and, after the last one, signals the epilogue;
 //   - warps 2..5: epilogue — tcgen05.ld of the 128 x N f32 accumulator into registers, staging
 //     through shared memory, then the same fused epilogues as the GEMV (gemv_epilogue: store,
@@ -72,6 +72,47 @@ __device__ __forceinline__ void tc_leave(TcShared *sh, int warp, int issued, int
     __syncthreads();
 }
 
+// Q8_0: the items of a row block that the epilogue left out because their sums are not finite.  A warp has the items that it had there
+// (the threads go round together); `part`: the segments' partial sums, where the row block is shared; pairs > 0: items of a row pair.
+template <class T>
+__device__ __noinline__ void tc_q8_redo(const GemvArgs *args, const float *stg, const float *part, int n_seg, int rb, int N, int pairs, int *known) {
+    const GemvArgs &a = *args;
+    const bool swiglu = a.epilogue == EPI_SWIGLU;
+    const int et = (int)threadIdx.x - 64, chunks = swiglu ? 8 : 16;
+    auto sum = [&](int row, int n) {
+        if (!part) return stg[row * (N + 1) + n];
+        float s = 0.f;
+        for (int i = 0; i < n_seg; ++i) s += __ldcg(part + ((size_t)i * N + n) * TC_BM + row);
+        return s;
+    };
+    if (pairs) {
+        for (int idx = et; idx < 64 * N; idx += 128) {
+            const int j = idx / N, n = idx - j * N, p = rb * 64 + j;
+            const bool mine = p < pairs && n < a.n_tok;
+            float v[2] = {0.f, 0.f};
+            if (mine) { v[0] = sum(swiglu ? j : 2 * j, n); v[1] = sum(swiglu ? 64 + j : 2 * j + 1, n); }
+            const bool odd = tc_q8_odd<2>(v);
+            tc_q8_mend<2>(a, odd, n, swiglu ? p : 2 * p, a.out, swiglu ? a.di + p : 2 * p + 1, v, known + n);
+            if (odd) gemv_epilogue<T>(a, p, n, v[0], v[1]);
+        }
+        return;
+    }
+    for (int idx = et; idx < chunks * N; idx += 128) {
+        const int c = idx % chunks, n = idx / chunks, first = rb * (8 * chunks) + 8 * c;
+        const bool mine = n < a.n_tok && first + 8 <= (swiglu ? a.di : a.out);
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = mine && (i < 8 || swiglu) ? sum(i < 8 ? 8 * c + i : 64 + 8 * c + i - 8, n) : 0.f;
+        const bool odd = tc_q8_odd<16>(v);
+        if (swiglu) tc_q8_mend<16>(a, odd, n, first, a.di, a.di + first, v, known + n);
+        else tc_q8_mend<8>(a, odd, n, first, a.out, first + 4, v, known + n);
+        if (!odd) continue;
+        TcPre pre;
+        tc_prefetch<T>(a, n, first, pre);
+        tc_finish<T>(a, n, first, v, v + 8, pre);
+    }
+}
+
 // Persistent: grid = min(tiles, SMs); a tile is (row block of 128 rows = 64 pairs, K split); CTA c takes
 // tiles c, c + grid, ...  The shared-memory ring keeps running across tiles and the accumulator is
 // double-buffered in TMEM, so the epilogue of one tile overlaps the loads and MMAs of the next.
@@ -82,7 +123,7 @@ __device__ __forceinline__ void tc_leave(TcShared *sh, int warp, int issued, int
 // 8B shape, 16 sequences: 5.13 -> 3.87 ms per round against the mma.sync kernel (28672 x 4096 in 34 us, its bytes 20).
 template <class T, bool Q8>
 __global__ void __launch_bounds__(Q8 ? TQ_THREADS : TC_THREADS, 1)
-gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_x,
+gemm_tc_kernel(const __grid_constant__ GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_x,
                int n_pairs, int N, int n_stages, int units_per_cta, int max_seg, int vec, uint32_t idesc, float *ws,
                unsigned *tickets, uint32_t *status) {
     extern __shared__ unsigned char smem_raw[];
@@ -119,11 +160,11 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             tc_mbar_init(tc_smem(&sh->a_empty[i]), 1);
         }
         tc_mbar_init(tc_smem(&sh->drain), 1);
-        for (int i = 0; Q8 && i < 64; ++i) sh->known[i] = TQ_UNKNOWN;
         sh->abort_flag = 0;
         sh->last = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (Q8 && tid >= 64 && tid < 128) sh->known[tid - 64] = TQ_UNKNOWN;
     if (warp == 1) {  // TMEM allocation is a warp-wide operation
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&sh->tmem_base)), "r"(tm_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -197,7 +238,8 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
         uint32_t phase = 0;
         [[maybe_unused]] int at = 0;  // Q8_0: the ring in tensor memory
         [[maybe_unused]] uint32_t at_phase = 0;
-        for (int u = u_begin; u < u_end && !sh->abort_flag; ++ti) {
+        bool stop = false;
+        for (int u = u_begin; u < u_end; ++ti) {
             const int kb1 = Q8 ? kb0 + 1 : min(nkb, kb0 + (u_end - u));  // Q8_0: every unit has an accumulator of its own
             const int ab = ti & 1;
             // the epilogue must have drained this accumulator (two tiles ago)
@@ -212,6 +254,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                 if (!tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag)) {
                     if (lane == 0) atomicOr(status, 4u);
                     sh->abort_flag = 1;
+                    stop = true;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -235,6 +278,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                     if (!ok) {
                         if (lane == 0) atomicOr(status, 4u);
                         sh->abort_flag = 1;
+                        stop = true;
                         break;
                     }
                 } else {
@@ -243,7 +287,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                 tc_warp_commit(empty0 + 8 * slot);  // the stage is free once these MMAs have read it
                 if (++slot == n_stages) { slot = 0; phase ^= 1u; }
             }
-            if (sh->abort_flag) break;                       // (one that lacks K blocks is never handed over)
+            if (stop) break;                                 // (one that lacks K blocks is never handed over)
             tc_warp_commit(tc_smem(&sh->tmem_full[ab]));     // accumulator complete
             u += kb1 - kb0;
             kb0 = Q8 && kb1 < nkb ? kb1 : 0;
@@ -372,6 +416,7 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
             }
             if (!all_ok) break;
             const int items = 64 * N;
+            [[maybe_unused]] bool odd = false;  // Q8_0: items left out, whose sums are not finite
             if (whole && vec) {
                 // (token, 8 outputs) items; residual vectors are fetched first, then everything is stored
                 const int chunks = swiglu ? 8 : 16;
@@ -386,37 +431,24 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                 for (int idx = et; idx < chunks * N; idx += 128, ++cnt) {
                     int c = idx % chunks, n = idx / chunks;
                     int first = swiglu ? rb * 64 + 8 * c : rb * TC_BM + 8 * c;
-                    const bool mine = n < a.n_tok && first + 8 <= (swiglu ? a.di : a.out);
-                    if (!Q8 && !mine) continue;
+                    if (!(n < a.n_tok && first + 8 <= (swiglu ? a.di : a.out))) continue;
                     float v[16];  // 8 outputs (SwiGLU: their gates, then their ups)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         v[i] = stg[(8 * c + i) * (N + 1) + n];
                         v[8 + i] = swiglu ? stg[(64 + 8 * c + i) * (N + 1) + n] : 0.f;
                     }
-                    if constexpr (Q8) {  // (16 * N and 8 * N items: the threads go round together)
-                        int known = sh->known[n];
-                        if (swiglu) tc_q8_mend<16>(a, mine, n, first, a.di, a.di + first, v, known);
-                        else tc_q8_mend<8>(a, mine, n, first, a.out, first + 4, v, known);
-                        if (!mine) continue;
-                        if (known) sh->known[n] = known;
-                    }
+                    if (Q8 && tc_q8_odd<16>(v)) { odd = true; continue; }
                     tc_finish<T>(a, n, first, v, v + 8, pre[cnt]);
                 }
             } else if (whole) {
                 for (int idx = et; idx < items; idx += 128) {
                     int j = idx / N, n = idx - j * N;
                     int p = rb * 64 + j;
-                    const bool mine = p < n_pairs && n < a.n_tok;
-                    if (!Q8 && !mine) continue;
+                    if (p >= n_pairs || n >= a.n_tok) continue;
                     int ra = swiglu ? j : 2 * j, rb2 = swiglu ? 64 + j : 2 * j + 1;
                     float v[2] = {stg[ra * (N + 1) + n], stg[rb2 * (N + 1) + n]};
-                    if constexpr (Q8) {
-                        int known = sh->known[n];
-                        tc_q8_mend<2>(a, mine, n, swiglu ? p : 2 * p, a.out, swiglu ? a.di + p : 2 * p + 1, v, known);
-                        if (!mine) continue;
-                        if (known) sh->known[n] = known;
-                    }
+                    if (Q8 && tc_q8_odd<2>(v)) { odd = true; continue; }
                     gemv_epilogue<T>(a, p, n, v[0], v[1]);
                 }
             } else {
@@ -485,17 +517,11 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                         for (int idx = et; idx < 8 * N; idx += 128) {
                             const int c = idx & 7, n = idx >> 3;
                             const int first = rb * 64 + 8 * c;
-                            const bool mine = n < a.n_tok && first + 8 <= a.di;
-                            if (!Q8 && !mine) continue;
+                            if (!(n < a.n_tok && first + 8 <= a.di)) continue;
                             float v[16];  // gates, ups
-                            const float *r = tile0 + (size_t)(mine ? n : 0) * TC_BM + 8 * c;
+                            const float *r = tile0 + (size_t)n * TC_BM + 8 * c;
                             merge2(r, r + 64, v, v + 8);
-                            if constexpr (Q8) {
-                                int known = sh->known[n];
-                                tc_q8_mend<16>(a, mine, n, first, a.di, a.di + first, v, known);
-                                if (!mine) continue;
-                                if (known) sh->known[n] = known;
-                            }
+                            if (Q8 && tc_q8_odd<16>(v)) { odd = true; continue; }
                             TcPre pre;
                             tc_finish<T>(a, n, first, v, v + 8, pre);
                         }
@@ -506,27 +532,25 @@ gemm_tc_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, cons
                             const int first = rb * TC_BM + 8 * c;
                             const bool rows_ok = first + 8 <= a.out;
                             const bool v0 = rows_ok && n0 < a.n_tok, v1 = rows_ok && n1 < a.n_tok && idx + 128 < 16 * N;
-                            if (!Q8 && !v0 && !v1) continue;
+                            if (!v0 && !v1) continue;
                             TcPre pre0, pre1;
                             if (v0) tc_prefetch<T>(a, n0, first, pre0);
                             if (v1) tc_prefetch<T>(a, n1, first, pre1);
                             float o0[8], o1[8];
-                            const float *r0 = tile0 + (size_t)(v0 ? n0 : v1 ? n1 : 0) * TC_BM + 8 * c;
-                            const float *r1 = tile0 + (size_t)(v1 ? n1 : v0 ? n0 : 0) * TC_BM + 8 * c;
+                            const float *r0 = tile0 + (size_t)(v0 ? n0 : n1) * TC_BM + 8 * c;
+                            const float *r1 = tile0 + (size_t)(v1 ? n1 : n0) * TC_BM + 8 * c;
                             merge2(r0, r1, o0, o1);
-                            if constexpr (Q8) {
-                                int k0 = sh->known[n0], k1 = sh->known[n1];
-                                tc_q8_mend<8>(a, v0, n0, first, a.out, first + 4, o0, k0);
-                                tc_q8_mend<8>(a, v1, n1, first, a.out, first + 4, o1, k1);
-                                if (v0 && k0) sh->known[n0] = k0;
-                                if (v1 && k1) sh->known[n1] = k1;
-                            }
-                            if (v0) tc_finish<T>(a, n0, first, o0, zero8, pre0);
-                            if (v1) tc_finish<T>(a, n1, first, o1, zero8, pre1);
+                            const bool odd0 = Q8 && v0 && tc_q8_odd<8>(o0), odd1 = Q8 && v1 && tc_q8_odd<8>(o1);
+                            if (v0 && !odd0) tc_finish<T>(a, n0, first, o0, zero8, pre0);
+                            if (v1 && !odd1) tc_finish<T>(a, n1, first, o1, zero8, pre1);
+                            odd = odd || odd0 || odd1;
                         }
                     }
                 }
             }
+            if constexpr (Q8)
+                if (__any_sync(0xffffffffu, odd))
+                    tc_q8_redo<T>(&a, stg, whole ? nullptr : ws + (size_t)rb * max_seg * N * TC_BM, n_seg, rb, N, whole && !vec ? n_pairs : 0, sh->known);
             asm volatile("bar.sync 2, 128;" ::: "memory");  // staging buffer is reused by the next tile
         }
     }
@@ -655,10 +679,12 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
         const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]);
         const uint64_t desc0 = tc_desc(tc_smem(smem));
         uint32_t phase = 0;
+        bool stop = false;
         for (int j = 0, slot = 0; j < n_units; ++j) {
             if (!tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag)) {
                 if (lane == 0) atomicOr(status, 4u);
                 sh->abort_flag = 1;
+                stop = true;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -667,7 +693,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
             tc_warp_commit(empty0 + 8 * slot);
             if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
-        if (!sh->abort_flag) tc_warp_commit(tc_smem(&sh->tmem_full[0]));  // (an accumulator that lacks K blocks is never handed over)
+        if (!stop) tc_warp_commit(tc_smem(&sh->tmem_full[0]));  // (an accumulator that lacks K blocks is never handed over)
     } else if (warp >= 2) {
         ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[0]), 0u, &sh->abort_flag));  // (the loads take the whole warp)
         if (!ok) {

@@ -188,21 +188,27 @@ __device__ __noinline__ int tc_q8_slow(const int8_t *q, const __half *s, const _
     }
     return known;
 }
+template <int CNT>
+__device__ __forceinline__ bool tc_q8_odd(const float *v) {  // whether one of them is not finite
+    float z[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) z[i & 1] = fmaf(v[i], 0.f, z[i & 1]);  // 0, or NaN
+    return z[0] + z[1] != 0.f;
+}
 // Replaces the sums of token n that are not finite (`mine`: the lane has a token).  v[i]: weight row row0 + i (below lim0), from CNT / 2
 // on row1 + i - CNT / 2 (below a.out).  Lanes with the same token (no more than 128 / CNT of them; one of 64) have theirs done together.
 // `known` stays with the token.  All lanes of the warp come here.
 template <int CNT>
-__device__ __forceinline__ void tc_q8_mend(const GemvArgs &a, bool mine, int n, int row0, int lim0, int row1, float *v, int &known) {
-    float z = 0.f;
-#pragma unroll
-    for (int i = 0; i < CNT; ++i) z = fmaf(v[i], 0.f, z);  // 0, or NaN
-    const bool todo = mine && z != 0.f && known != TQ_NAN;
-    if (!__any_sync(0xffffffffu, todo)) return;
+__device__ __forceinline__ void tc_q8_mend(const GemvArgs &a, bool mine, int n, int row0, int lim0, int row1, float *v, int *known) {
+    const bool odd = mine && tc_q8_odd<CNT>(v);
+    if (!__any_sync(0xffffffffu, odd)) return;
+    const int was = mine ? *known : TQ_UNKNOWN;
     float w[CNT];
 #pragma unroll
     for (int i = 0; i < CNT; ++i) w[i] = v[i];
-    known = tc_q8_slow<CNT>(reinterpret_cast<const int8_t *>(a.w), reinterpret_cast<const __half *>(a.w_scales), reinterpret_cast<const __half *>(a.x), a.stride_x, a.in,
-                            a.out, todo, n, row0, lim0, row1, known, w);
+    const int now = tc_q8_slow<CNT>(reinterpret_cast<const int8_t *>(a.w), reinterpret_cast<const __half *>(a.w_scales), reinterpret_cast<const __half *>(a.x), a.stride_x, a.in,
+                            a.out, odd && was != TQ_NAN, n, row0, lim0, row1, was, w);
+    if (mine && now != was) *known = now;
 #pragma unroll
     for (int i = 0; i < CNT; ++i) v[i] = w[i];
 }
