@@ -23,7 +23,14 @@
 
 namespace lcu {
 
-constexpr int TP_THREADS = 320;
+constexpr int TP_THREADS = 320, TP_SPAN_THREADS = 576;
+// The tensor pipe cuts a sum off where it would have to round it, so the error of a sum grows with the products of one accumulator
+// (4096 in a row: 4.9e-6 of the result, 14336: 1.7e-5; f16 rounds by 2e-4).  Where smaller launches divide K among CTAs, so that
+// their sums are shorter, this kernel cuts K into as many spans with an accumulator each, which are added up, rounded: two of tiles
+// of 128 rows fit into tensor memory side by side; more of them, or of larger tiles, are taken one by one into registers, by twice
+// the epilogue warps with 64 sums each (997 tokens of the 8B shape, all in spans of 1024: 14.8 -> 15.1 ms; with 128 sums in half
+// of the warps 16.4).
+enum { TP_PLAIN, TP_SPANS, TP_Q8 };
 constexpr int TP_BM = 128;                       // tokens per CTA
 constexpr int TP_A_BYTES = TP_BM * TC_BK * 2;
 constexpr int TP_STAGES = 7;
@@ -35,9 +42,11 @@ constexpr int TP_STAGES = 7;
 // MMAs 512; measured 830.  28672 x 4096 with 500 tokens in 170 us (0.69 PFLOP/s, counting each product once), eight passes of the
 // mma.sync kernel 1080 us; 500 tokens of the 8B shape 67.7 -> 16.5 ms.
 constexpr int TPQ_STAGES = 5, TPQ_GROUPS = 3;
-constexpr int TPQ_THREADS = TP_THREADS + 256 + 32;
+constexpr int TPQ_CONVERT = 320;                          // first converting thread
+constexpr int TPQ_THREADS = TPQ_CONVERT + 256 + 32;
 constexpr int TPQ_ROWS = 64;                              // weight rows of a CTA
 constexpr int TPQ_Q_BYTES = TPQ_ROWS * TQ_K, TPQ_G_BYTES = TPQ_Q_BYTES + TPQ_ROWS * (TQ_K / 32) * 2;
+template <int MODE> constexpr int tp_threads() { return MODE == TP_Q8 ? TPQ_THREADS : MODE == TP_SPANS ? TP_SPAN_THREADS : TP_THREADS; }
 constexpr int TP_COLS = 256;                     // TMEM columns of one accumulator
 
 struct TpShared {
@@ -65,6 +74,7 @@ __device__ __forceinline__ void tp_commit_both(uint32_t bar) {
                  " @e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
                  ::"r"(bar), "h"((unsigned short)3) : "memory");
 }
+__device__ __forceinline__ uint32_t tp_add(uint32_t x, uint32_t y) { return __float_as_uint(__uint_as_float(x) + __uint_as_float(y)); }
 __device__ __forceinline__ void tp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -86,14 +96,16 @@ __device__ __forceinline__ bool tp_wait_both(uint32_t bar, uint32_t parity, vola
 }
 
 // NT: weight rows of a tile (a multiple of 64; SwiGLU: NT / 2 gate rows, then their NT / 2 up rows)
-template <class T, bool Q8>
-__global__ void __launch_bounds__(Q8 ? TPQ_THREADS : TP_THREADS, 1) __cluster_dims__(2, 1, 1)
+template <class T, int MODE>
+__global__ void __launch_bounds__(tp_threads<MODE>(), 1) __cluster_dims__(2, 1, 1)
 gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_x, int NT,
-                 int n_mt, int n_tiles, uint32_t idesc, uint32_t *status) {
+                 int n_mt, int n_tiles, int span, uint32_t idesc, uint32_t *status) {
+    constexpr bool Q8 = MODE == TP_Q8;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (tc_smem(smem_raw) & 1023u)) & 1023u);
     const int half = NT / 2;
     constexpr int STAGES = Q8 ? TPQ_STAGES : TP_STAGES, COPIES = Q8 ? 2 : 1;
+    const int SPAN = Q8 ? TQ_K / TC_BK : span;
     const int stage_bytes = TP_A_BYTES + COPIES * half * 128;
     unsigned char *raw = smem + (size_t)STAGES * (TP_A_BYTES + (Q8 ? 2 * TPQ_ROWS : TP_COLS / 2) * 128);  // Q8_0: bytes and scales
     TpShared *sh = reinterpret_cast<TpShared *>(raw + (Q8 ? TPQ_GROUPS * TPQ_G_BYTES : 0));
@@ -112,7 +124,7 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
         }
         for (int i = 0; i < 2; ++i) {
             tc_mbar_init(tc_smem(&sh->tmem_full[i]), 1);
-            tc_mbar_init(tc_smem(&sh->tmem_empty[i]), 16);  // a lane of every epilogue warp of both CTAs
+            tc_mbar_init(tc_smem(&sh->tmem_empty[i]), MODE == TP_SPANS ? 32 : 16);  // a lane of every epilogue warp of both CTAs
         }
         for (int i = 0; Q8 && i < TPQ_GROUPS; ++i) {
             tc_mbar_init(tc_smem(&sh->g_full[i]), 1);
@@ -182,11 +194,10 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
             // ---------------- MMA issuer
             const uint32_t full0 = tc_smem(&sh->full[0]), empty0 = tc_smem(&sh->empty[0]);
             const uint64_t desc0 = tc_desc(tc_smem(smem));
-            int ti = 0, slot = 0;  // accumulators taken: one per tile, Q8_0: per group of four K blocks
+            int ti = 0, slot = 0, kb = 0;  // accumulators taken: one per span
             bool stop = false;
             uint32_t phase = 0;
-            const int span = Q8 ? 4 : nkb;
-            const int n_acc = pair < n_tiles ? (n_tiles - pair + n_pairs - 1) / n_pairs * (nkb / span) : 0;
+            const int n_acc = pair < n_tiles ? (n_tiles - pair + n_pairs - 1) / n_pairs * (MODE == TP_PLAIN ? 1 : (nkb + SPAN - 1) / SPAN) : 0;
             for (; ti < n_acc && !stop; ++ti) {
                 const int ab = ti & 1;
                 if (!tc_warp_wait(tc_smem(&sh->tmem_empty[ab]), ((uint32_t)(ti >> 1) & 1u) ^ 1u, &sh->abort_flag)) {
@@ -197,7 +208,9 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d_tmem = tmem + (uint32_t)(ab * TP_COLS);
-                for (int kb = 0; kb < span; ++kb) {
+                const int k0 = kb, k1 = Q8 ? kb + SPAN : MODE == TP_PLAIN ? nkb : min(nkb, kb + SPAN);
+                const int k2 = MODE == TP_PLAIN && span < nkb ? span : 0;  // from here on in a second accumulator
+                for (; kb < k1; ++kb) {
                     if (!(Q8 ? tp_wait_both(full0 + 8 * slot, phase, &sh->abort_flag) : tc_warp_wait(full0 + 8 * slot, phase, &sh->abort_flag))) {
                         if (lane == 0) atomicOr(status, 4u);
                         sh->abort_flag = 1;
@@ -206,11 +219,12 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4), db = da + (TP_A_BYTES >> 4);
-                    tp_mma4(d_tmem, da, db, idesc, kb > 0 ? 1u : 0u);
+                    tp_mma4(MODE == TP_PLAIN && k2 && kb >= k2 ? d_tmem + NT : d_tmem, da, db, idesc, kb > k0 && (MODE != TP_PLAIN || kb != k2));
                     if (Q8) tp_mma4(d_tmem, da, db + (uint64_t)((half * 128) >> 4), idesc, 1u);
                     tp_commit_both(empty0 + 8 * slot);
                     if (++slot == STAGES) { slot = 0; phase ^= 1u; }
                 }
+                if (kb == nkb) kb = 0;
                 if (!stop) tp_commit_both(tc_smem(&sh->tmem_full[ab]));  // (an accumulator that lacks K blocks is never handed over)
             }
         }
@@ -237,11 +251,11 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 if (++slot == TPQ_GROUPS) { slot = 0; phase ^= 1u; }
             }
         }
-    } else if (Q8 && warp >= TP_THREADS / 32) {
+    } else if (Q8 && warp >= TPQ_CONVERT / 32) {
         // ---------------- Q8_0: the converting warps work in pairs, one stage of a group each (a row per thread): the fence and the
         // hand-over of a stage take longer than its arithmetic, and so they run side by side
         if constexpr (Q8) {
-            const int u = (warp - TP_THREADS / 32) >> 1, row = (tid - TP_THREADS) & (TPQ_ROWS - 1);
+            const int u = (warp - TPQ_CONVERT / 32) >> 1, row = (tid - TPQ_CONVERT) & (TPQ_ROWS - 1);
             const uint32_t empty0 = tc_smem(&sh->empty[0]), full0_leader = tp_in_leader(tc_smem(&sh->full[0]));
             int slot = u, gs = 0;
             uint32_t phase = 1, g_phase = 0;
@@ -285,131 +299,160 @@ gemm_pair_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, co
                 sh->abort_flag = 1;
             }
         }
-    } else if (Q8 && warp >= 2) {
-        // ---------------- Q8_0: epilogue.  A thread has one token and 64 outputs (SwiGLU: 32 gates, then their ups): sums over the groups
-        if constexpr (Q8) {
+    } else if (MODE == TP_PLAIN && warp >= 2) {
+        // ---------------- epilogue: a thread has one token; the two warps of a quadrant take half of the columns each
+        if constexpr (MODE == TP_PLAIN) {
             const int q = warp & 3, h = (warp - 2) >> 2;
-            const int c_a = swiglu ? h * 32 : h * 64, c_b = swiglu ? TPQ_ROWS + h * 32 : c_a + 32;
-            int ti = 0, known = TQ_UNKNOWN, known_n = -1;
-            bool ok = true;
-            grid_dep_wait();
-            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                const int nt = tile / n_mt, mt = tile - nt * n_mt;
-                const int n = mt * 2 * TP_BM + rank * TP_BM + q * 32 + lane;
-                float sum[64];
-#pragma unroll
-                for (int i = 0; i < 64; ++i) sum[i] = 0.f;
-                for (int kb = 0; kb < nkb && ok; kb += 4, ++ti) {
-                    const int ab = ti & 1;
-                    ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag));
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * TP_COLS);
-#pragma unroll
-                    for (int c = 0; c < 64; c += 16) {
-                        uint32_t r[16];
-                        tc_ld16(acc + (uint32_t)(c < 32 ? c_a + c : c_b + c - 32), r);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(r[i]);
-                    }
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0)
-                        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
+            int ti = 0;
+            grid_dep_wait();  // residual rows and the round descriptor are earlier kernels'
+            for (int tile = pair; tile < n_tiles; tile += n_pairs, ++ti) {
+                const int mt = tile % n_mt, nt = tile / n_mt;
+                const int ab = ti & 1;
+                if (!__all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag))) {  // (the loads take the whole warp)
+                    if (lane == 0) atomicOr(status, 4u);
+                    sh->abort_flag = 1;
+                    break;
                 }
-                if (!ok) break;
-                const int r0 = nt * step + c_a;
-                if (n != known_n) { known = TQ_UNKNOWN; known_n = n; }
-                tc_q8_mend<64>(a, n < a.n_tok, n, r0, swiglu ? a.di : a.out, swiglu ? a.di + r0 : r0 + 32, sum, &known);
-                if (n >= a.n_tok) continue;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int n = mt * 2 * TP_BM + rank * TP_BM + q * 32 + lane;
+                const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * TP_COLS);
                 if (swiglu) {
+                    for (int c0 = h * (half / 2); c0 < (h + 1) * (half / 2); c0 += 16) {
+                        uint32_t g[16], u[16];
+                        tc_ld16(acc + (uint32_t)c0, g);
+                        tc_ld16(acc + (uint32_t)(half + c0), u);
+                        if (span < nkb) {
+                            uint32_t g2[16], u2[16];
+                            tc_ld16(acc + (uint32_t)(NT + c0), g2);
+                            tc_ld16(acc + (uint32_t)(NT + half + c0), u2);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        const int first = nt * step + c_a + c;
-                        if (first + 8 > a.di) continue;
+                            for (int i = 0; i < 16; ++i) { g[i] = tp_add(g[i], g2[i]); u[i] = tp_add(u[i], u2[i]); }
+                        }
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                         TcPre pre;
-                        tc_finish<T>(a, n, first, sum + c, sum + 32 + c, pre);
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 64; c += 16) {
-                        const int first = nt * step + c_a + c;
-                        TcPre pre[2];
-#pragma unroll
-                        for (int k = 0; k < 2; ++k)
-                            if (first + 8 * k + 8 <= a.out) tc_prefetch<T>(a, n, first + 8 * k, pre[k]);
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
-                            if (first + 8 * k + 8 > a.out) continue;
-                            tc_finish<T>(a, n, first + 8 * k, sum + c + 8 * k, sum + c + 8 * k, pre[k]);
+                            const int first = nt * step + c0 + 8 * k;
+                            if (n >= a.n_tok || first + 8 > a.di) continue;
+                            float v[8], w[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) { v[i] = __uint_as_float(g[8 * k + i]); w[i] = __uint_as_float(u[8 * k + i]); }
+                            tc_finish<T>(a, n, first, v, w, pre);
+                        }
+                    }
+                } else {
+                    for (int c0 = h * half; c0 < (h + 1) * half; c0 += 32) {
+                        const int first = nt * step + c0;
+                        TcPre pre[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (n < a.n_tok && first + 8 * k + 8 <= a.out) tc_prefetch<T>(a, n, first + 8 * k, pre[k]);
+                        uint32_t r[32];
+                        tc_ld16(acc + (uint32_t)c0, r);
+                        tc_ld16(acc + (uint32_t)(c0 + 16), r + 16);
+                        if (span < nkb) {
+                            uint32_t r2[32];
+                            tc_ld16(acc + (uint32_t)(NT + c0), r2);
+                            tc_ld16(acc + (uint32_t)(NT + c0 + 16), r2 + 16);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) r[i] = tp_add(r[i], r2[i]);
+                        }
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (n >= a.n_tok || first + 8 * k + 8 > a.out) continue;
+                            float v[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[8 * k + i]);
+                            tc_finish<T>(a, n, first + 8 * k, v, v, pre[k]);
                         }
                     }
                 }
-            }
-            if (!ok) {
-                if (lane == 0) atomicOr(status, 4u);
-                sh->abort_flag = 1;
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
             }
         }
     } else if (warp >= 2) {
-        // ---------------- epilogue: a thread has one token; the two warps of a quadrant take half of the columns each
+        // ---------------- epilogue of spans: a thread has one token; the four warps of a quadrant (Q8_0: two) share the columns and add
+        // the spans up.
+        // The first half of the sums and the second (SwiGLU: gates and their ups) are `len_a` and `len_b` columns from c_a and c_b on.
+        constexpr int COLS = 64, WPQ = Q8 ? 2 : 4;  // most columns of a thread, warps of a quadrant
+        const int cols = NT / WPQ;
         const int q = warp & 3, h = (warp - 2) >> 2;
+        const int c_a = swiglu ? h * (cols / 2) : h * cols, c_b = swiglu ? half + c_a : c_a + COLS / 2;
+        const int len_a = swiglu ? cols / 2 : min(cols, COLS / 2), len_b = cols - len_a;
         int ti = 0;
+        [[maybe_unused]] int known = TQ_UNKNOWN, known_n = -1;
+        bool ok = true;
         grid_dep_wait();  // residual rows and the round descriptor are earlier kernels'
-        for (int tile = pair; tile < n_tiles; tile += n_pairs, ++ti) {
-            const int mt = tile % n_mt, nt = tile / n_mt;
-            const int ab = ti & 1;
-            if (!__all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag))) {  // (the loads take the whole warp)
-                if (lane == 0) atomicOr(status, 4u);
-                sh->abort_flag = 1;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int nt = tile / n_mt, mt = tile - nt * n_mt;
             const int n = mt * 2 * TP_BM + rank * TP_BM + q * 32 + lane;
-            const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * TP_COLS);
-            if (swiglu) {
-                for (int c0 = h * (half / 2); c0 < (h + 1) * (half / 2); c0 += 16) {
-                    uint32_t g[16], u[16];
-                    tc_ld16(acc + (uint32_t)c0, g);
-                    tc_ld16(acc + (uint32_t)(half + c0), u);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    TcPre pre;
+            float sum[COLS];
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const int first = nt * step + c0 + 8 * k;
-                        if (n >= a.n_tok || first + 8 > a.di) continue;
-                        float v[8], w[8];
+            for (int i = 0; i < COLS; ++i) sum[i] = 0.f;
+            for (int kb = 0; kb < nkb && ok; kb += SPAN, ++ti) {
+                const int ab = ti & 1;
+                ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&sh->tmem_full[ab]), (uint32_t)(ti >> 1) & 1u, &sh->abort_flag));  // (the loads take the whole warp)
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ab * TP_COLS);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) { v[i] = __uint_as_float(g[8 * k + i]); w[i] = __uint_as_float(u[8 * k + i]); }
-                        tc_finish<T>(a, n, first, v, w, pre);
+                for (int c = 0; c < COLS; c += 16) {
+                    const int at = c % (COLS / 2), len = c < COLS / 2 ? len_a : len_b;
+                    if (!Q8 && at >= len) continue;
+                    uint32_t r[16];
+                    if (Q8 || at + 16 <= len) {
+                        tc_ld16(acc + (uint32_t)((c < COLS / 2 ? c_a : c_b) + at), r);
+                    } else {  // (24 columns)
+                        tc_ld8(acc + (uint32_t)((c < COLS / 2 ? c_a : c_b) + at), r);
+#pragma unroll
+                        for (int i = 8; i < 16; ++i) r[i] = 0u;
                     }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(r[i]);
                 }
-            } else {
-                for (int c0 = h * half; c0 < (h + 1) * half; c0 += 32) {
-                    const int first = nt * step + c0;
-                    TcPre pre[4];
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
+            }
+            if (!ok) break;
+            const int first = nt * step + c_a;
+            if constexpr (Q8) {
+                if (n != known_n) { known = TQ_UNKNOWN; known_n = n; }
+                tc_q8_mend<COLS>(a, n < a.n_tok, n, first, swiglu ? a.di : a.out, swiglu ? a.di + first : first + COLS / 2, sum, &known);
+            }
+            if (n >= a.n_tok) continue;
+            if (swiglu) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (n < a.n_tok && first + 8 * k + 8 <= a.out) tc_prefetch<T>(a, n, first + 8 * k, pre[k]);
-                    uint32_t r[32];
-                    tc_ld16(acc + (uint32_t)c0, r);
-                    tc_ld16(acc + (uint32_t)(c0 + 16), r + 16);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int c = 0; c < COLS / 2; c += 8) {
+                    if (c >= len_a || first + c + 8 > a.di) continue;
+                    TcPre pre;
+                    tc_finish<T>(a, n, first + c, sum + c, sum + COLS / 2 + c, pre);
+                }
+            } else {  // (c_b follows the first half)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (n >= a.n_tok || first + 8 * k + 8 > a.out) continue;
-                        float v[8];
+                for (int c = 0; c < COLS; c += 16) {
+                    if (c >= cols) continue;
+                    TcPre pre[2];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[8 * k + i]);
-                        tc_finish<T>(a, n, first + 8 * k, v, v, pre[k]);
-                    }
+                    for (int k = 0; k < 2; ++k)
+                        if (first + c + 8 * k + 8 <= a.out) tc_prefetch<T>(a, n, first + c + 8 * k, pre[k]);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        if (first + c + 8 * k + 8 <= a.out) tc_finish<T>(a, n, first + c + 8 * k, sum + c + 8 * k, sum + c + 8 * k, pre[k]);
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tp_in_leader(tc_smem(&sh->tmem_empty[ab]))) : "memory");
+        }
+        if (!ok) {
+            if (lane == 0) atomicOr(status, 4u);
+            sh->abort_flag = 1;
         }
     }
     // ---------------- tail: both CTAs are done with each other's barriers and accumulators
@@ -457,8 +500,9 @@ bool gemm_pair_takes(const GemvArgs &a) {
     return 2 * n_mt * ((rows + NT - 1) / NT) > pairs;
 }
 
-template <class T, bool Q8>
-static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, bool dry) {
+template <class T, int MODE>
+static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, bool dry, int pieces) {
+    constexpr bool Q8 = MODE == TP_Q8;
     static std::mutex mu;
     static std::map<int, bool> done;
     int dev = 0;
@@ -466,7 +510,7 @@ static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!done[dev]) {
-            LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<T, Q8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes<Q8>()));
+            LCU_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes<Q8>()));
             done[dev] = true;
         }
     }
@@ -482,22 +526,33 @@ static int tp_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32
     if (rc) return rc;
     const uint32_t fmt = dt == LCU_BF16 ? 1u : 0u;
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(2 * TP_BM >> 4) << 24);
-    const int tiles = n_mt * n_nt;
+    const int tiles = n_mt * n_nt, nkb = a.in / TC_BK;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);
-    LCU_CHECK_CUDA(launch_kernel(gemm_pair_kernel<T, Q8>, dim3(grid), dim3(Q8 ? TPQ_THREADS : TP_THREADS), tp_smem_bytes<Q8>(), s, pdl, a, mw, Q8 ? ms : mw, mx, NT, n_mt, tiles, idesc, status));
+    LCU_CHECK_CUDA(launch_kernel(gemm_pair_kernel<T, MODE>, dim3(grid), dim3(tp_threads<MODE>()), tp_smem_bytes<Q8>(), s, pdl, a, mw, Q8 ? ms : mw, mx, NT, n_mt, tiles,
+                                 (nkb + pieces - 1) / pieces, idesc, status));
     g_linear_last_ctas = grid;
     return LCU_OK;
 }
 
-int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status) {
-    if (a.w_q8) return tp_launch<__half, true>(a, dt, s, pdl, status, false);
-    return dt == LCU_F16 ? tp_launch<__half, false>(a, dt, s, pdl, status, false) : tp_launch<__nv_bfloat16, false>(a, dt, s, pdl, status, false);
+template <class T>
+static int tp_16bit(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, bool dry, int pieces) {
+    const int rows = a.epilogue == EPI_SWIGLU ? 2 * a.di : a.out, n_mt = (a.n_tok + 2 * TP_BM - 1) / (2 * TP_BM);
+    if (dry || pieces <= (tp_tile(n_mt, rows, sm_count() / 2) <= TP_COLS / 2 ? 2 : 1)) {
+        const int rc = tp_launch<T, TP_PLAIN>(a, dt, s, pdl, status, dry, pieces);
+        if (rc || !dry) return rc;
+    }
+    return tp_launch<T, TP_SPANS>(a, dt, s, pdl, status, dry, pieces);
+}
+
+int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, int pieces) {
+    if (a.w_q8) return tp_launch<__half, TP_Q8>(a, dt, s, pdl, status, false, 1);
+    return dt == LCU_F16 ? tp_16bit<__half>(a, dt, s, pdl, status, false, pieces) : tp_16bit<__nv_bfloat16>(a, dt, s, pdl, status, false, pieces);
 }
 
 int gemm_pair_warm(int dt, bool q8) {
     GemvArgs a{};
-    if (q8) return tp_launch<__half, true>(a, dt, nullptr, false, nullptr, true);
-    return dt == LCU_F16 ? tp_launch<__half, false>(a, dt, nullptr, false, nullptr, true) : tp_launch<__nv_bfloat16, false>(a, dt, nullptr, false, nullptr, true);
+    if (q8) return tp_launch<__half, TP_Q8>(a, dt, nullptr, false, nullptr, true, 1);
+    return dt == LCU_F16 ? tp_16bit<__half>(a, dt, nullptr, false, nullptr, true, 1) : tp_16bit<__nv_bfloat16>(a, dt, nullptr, false, nullptr, true, 1);
 }
 
 }  // namespace lcu

@@ -33,6 +33,7 @@ constexpr int TC_BM = 128;         // weight rows per CTA tile
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;
 
 constexpr int TC_MAX_STAGES = 12;
+constexpr int TC_LONG = 32;        // K blocks of an accumulator that show: 2048 products err by 2.4e-6, an 80th of f16's rounding
 
 // Q8_0 weights: 8 more warps turn a unit's weights into f16 pairs in tensor memory, from where the MMA takes them as its A operand
 // (lane = row); through shared memory they would cost it four times the bytes that HBM delivers.
@@ -598,7 +599,7 @@ __device__ __forceinline__ float4 tc_ld_dsmem4(uint32_t local_saddr, uint32_t ct
 template <class T>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                int N, int n_stages, int KS, uint32_t idesc, uint32_t *status) {
+                int N, int n_stages, int KS, int accs, uint32_t idesc, uint32_t *status) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (tc_smem(smem_raw) & 1023u)) & 1023u);
     const int stage_bytes = TC_A_BYTES + N * 128;
@@ -621,7 +622,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
     }
     const int kb0 = (int)((long)ks * nkb / KS), kb1 = (int)((long)(ks + 1) * nkb / KS);
     const int n_units = kb1 - kb0;
-    const int tm_cols = N < 32 ? 32 : N;
+    const int acc_cols = N < 32 ? 32 : N, tm_cols = accs * acc_cols, half = accs > 1 ? (n_units + 1) / 2 : n_units;  // K blocks of the first accumulator
 
     if (tid == 0) {
         for (int i = 0; i < n_stages; ++i) {
@@ -689,7 +690,7 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t da = desc0 + (uint64_t)((slot * stage_bytes) >> 4);
-            tc_warp_mma4(tmem, da, da + (TC_A_BYTES >> 4), idesc, j > 0 ? 1u : 0u);
+            tc_warp_mma4(j < half ? tmem : tmem + acc_cols, da, da + (TC_A_BYTES >> 4), idesc, j > 0 && j != half);
             tc_warp_commit(empty0 + 8 * slot);
             if (++slot == n_stages) { slot = 0; phase ^= 1u; }
         }
@@ -709,14 +710,28 @@ gemm_tck_kernel(const GemvArgs a, const __grid_constant__ CUtensorMap map_w, con
             // ---------------- accumulator columns [t0, t0 + NS) -> token-major staging tile
             const int q = warp & 3;
             const int row = q * 32 + lane;
-            for (int c0 = 0; c0 < NS; c0 += 16) {
-                uint32_t r[16];
+            for (int c0 = 0; c0 < NS; c0 += 32) {
+                uint32_t r[32];
+                const bool more = c0 + 16 < NS;
                 if (ok) {
-                    tc_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t0 + c0), r);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t0 + c0);
+                    tc_ld16(at, r);
+                    if (more) tc_ld16(at + 16, r + 16);
+                    if (half < n_units) {
+                        uint32_t r2[32];
+                        tc_ld16(at + acc_cols, r2);
+                        if (more) tc_ld16(at + acc_cols + 16, r2 + 16);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (i < 16 || more) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
+                    } else {
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    }
                 }
 #pragma unroll
-                for (int i = 0; i < 16; ++i) stg[(size_t)(c0 + i) * TCK_LD + row] = ok ? __uint_as_float(r[i]) : 0.f;
+                for (int i = 0; i < 32; ++i)
+                    if (i < 16 || more) stg[(size_t)(c0 + i) * TCK_LD + row] = ok ? __uint_as_float(r[i]) : 0.f;
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -857,7 +872,15 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
         if (!status) status = it->second;
     }
     if (dry) return gemm_pair_warm(dt, Q8);
-    if (gemm_pair_takes(a)) return gemm_pair_launch(a, dt, s, pdl, status);
+    // A sum is cut into no fewer pieces than CTAs would fill the GPU with (the tensor pipe's error grows with the products of one
+    // accumulator), however few CTAs the launch divides K among: the rest are accumulators of one CTA.  The stand-alone operator,
+    // which has no scratch, counts a block of 64 tokens.
+    const int row_blocks = (a.out / 2 + 63) / 64, tok_blocks = g_tc_ws ? (a.n_tok + 255) / 256 : 1;
+    int pieces = a.tiles ? 1 : sm_count() / (row_blocks * tok_blocks);
+    pieces = pieces > 8 ? 8 : pieces < 1 ? 1 : pieces;
+    while (pieces > 1 && a.in / TC_BK / pieces < 4) --pieces;
+    if (a.in / TC_BK < TC_LONG) pieces = 1;
+    if (gemm_pair_takes(a)) return gemm_pair_launch(a, dt, s, pdl, status, pieces);
     const int n_pairs = a.out / 2;
     const int sms = sm_count();
     const uint32_t fmt = dt == LCU_BF16 ? 1u : 0u;
@@ -943,7 +966,7 @@ static int tc_launch_t(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, bool
             attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = pdl ? 2 : 1;
-            LCU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tck_kernel<T>, a, mw, mx, N, st, KS, idesc_c, status));
+            LCU_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tck_kernel<T>, a, mw, mx, N, st, KS, KS < pieces && nkb_c / KS >= TC_LONG ? 2 : 1, idesc_c, status));
             g_linear_last_ctas = n_rb_c * KS * n_tb;
             return LCU_OK;
         }

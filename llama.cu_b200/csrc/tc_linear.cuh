@@ -371,7 +371,7 @@ inline bool tc_vec(const GemvArgs &a) {  // whether the 16-byte epilogues apply
 
 // 256 x up to 256 tiles on pairs of SMs for rounds of many tokens (gemm_pair.cu); the arguments are those of gemm_tc_launch.
 bool gemm_pair_takes(const GemvArgs &a);
-int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status);
+int gemm_pair_launch(const GemvArgs &a, int dt, cudaStream_t s, bool pdl, uint32_t *status, int pieces);  // pieces: of a sum
 int gemm_pair_warm(int dt, bool q8);
 
 }  // namespace lcu

@@ -19,12 +19,10 @@ def pair(L):
 
 
 @pytest.mark.parametrize("dt", [0, 1])
-@pytest.mark.parametrize("n", [1, 127, 129, 256, 257, 520])
+@pytest.mark.parametrize("n", [9, 127, 129, 256, 257, 520])
 @pytest.mark.parametrize("out,k", [(8, 64), (136, 512), (1000, 192), (4096, 448), (9480, 960)])
 @pytest.mark.parametrize("res", [False, True])
 def test_product(L, pair, dt, n, out, k, res):
-    if n <= 8:
-        n = 9  # fewer tokens go to the mma.sync kernel
     pair(1)
     tdt = L.torch_dtype(dt)
     g = torch.Generator(device=DEV)
@@ -40,6 +38,34 @@ def test_product(L, pair, dt, n, out, k, res):
     bound = want.abs() * 2.0 ** (-11 if dt == 0 else -8) + (x.double().abs() @ w.double().abs().T + 1) * (k + 1) * 2.0 ** -24
     assert bool(((y[:n].double() - want).abs() <= bound).all())
     assert bool((y[n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dt", [0, 1])
+@pytest.mark.parametrize("n,out,k", [(200, 6144, 4096), (300, 4096, 4096), (300, 4096, 14336), (1000, 2048, 8192), (520, 1024, 1088)])
+def test_sums(L, pair, dt, n, out, k):
+    """The tensor pipe cuts a sum off where it would have to round it: an error that grows with the products of one accumulator.  Sums
+    are cut into as many pieces as CTAs would fill the GPU with.  Seen by way of a residual that takes the rounded product away again."""
+    pair(1)
+    tdt = L.torch_dtype(dt)
+    g = torch.Generator(device=DEV)
+    g.manual_seed(k)
+    x = torch.randn(n, k, device=DEV, generator=g).to(tdt)
+    w = torch.randn(out, k, device=DEV, generator=g).mul_(0.02).to(tdt)
+    want = x.double() @ w.double().T
+    r = (-want).to(tdt)
+    y = torch.empty(n, out, device=DEV, dtype=tdt)
+    L.check(L.load_library().lcu_op_linear(y.data_ptr(), out, x.data_ptr(), k, w.data_ptr(), dt, r.data_ptr(), out, n, k, out, dt,
+                                           C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    err = y.double() - (want + r.double())
+    pieces = min(8, max(1, torch.cuda.get_device_properties(0).multi_processor_count // -(-out // 128)))
+    if k // 64 < 32:
+        pieces = 1
+    while pieces > 1 and k // 64 // pieces < 4:
+        pieces -= 1
+    steps = -(-k // 64 // pieces) * 4
+    # a step of 16 products cuts half a unit of 24 bits on average, of a sum that grows like a root: a third of one of the result; with 30 %
+    # to spare.  And y's own rounding, of a difference of 2^-12 (bf16: 2^-9)
+    assert float(err.norm() / want.norm()) < 1.3 * steps * 2.0 ** -24 / 3 + (2.0 ** -24 if dt == 0 else 2.0 ** -18)
 
 
 @pytest.mark.parametrize("act", [0, 1])
