@@ -1,5 +1,6 @@
 // Causal GQA attention over the KV cache for the tokens of one round.  Interface only.
 #pragma once
+#include "attention_plan.hpp"
 #include "common.cuh"
 
 namespace lcu {
@@ -58,7 +59,7 @@ int attn_prefill_launch(const AttnArgs &a, const void *groups_dev, int n_groups,
 
 // The same rounds on tcgen05 (attention_tc.cu): groups of up to attn_tc_group_tokens tokens, any number of pages.
 int attn_tc_group_tokens(int nh, int nkvh);
-bool attn_tc_takes(const KvGeom &g, int n_pages, const void *pool, unsigned longest);
+bool attn_tc_takes(const KvGeom &g, int n_pages, const void *pool);
 int attn_tc_launch(const AttnArgs &a, const void *groups_dev, int n_groups, int dt, cudaStream_t s, bool dry = false);
 
 // Appends k, v [seq, nkvh, dh] (strided) to linear caches at pos.. (the write half of

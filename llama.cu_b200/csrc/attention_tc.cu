@@ -394,10 +394,7 @@ static int at_launch(const AttnArgs &a, const void *groups, int n_groups, int dt
 
 int attn_tc_group_tokens(int nh, int nkvh) { return 256 / (nh / nkvh); }
 
-// longest: the longest context of the round.  A CTA starts and ends 3 us slower than one of the mma.sync kernel, which walks 64
-// positions in the time that this one takes for 256 (33 tokens of the 1B shape: 7.5 against 4.5 us per layer).
-bool attn_tc_takes(const KvGeom &g, int n_pages, const void *pool, unsigned longest) {
-    if (longest <= 128 && tuning().attn_tc < 2) return false;
+bool attn_tc_takes(const KvGeom &g, int n_pages, const void *pool) {
     // blocks of a page are one coordinate of the map (32 bits); the map's base is 16-byte aligned
     return tuning().attn_tc && tc_encode_fn() && (uintptr_t)pool % 16 == 0 && (unsigned long long)n_pages * g.n_layers * 2 * g.nkvh < (1ull << 31);
 }

@@ -90,49 +90,19 @@ static int attn_tiles(const lcu_ctx *c, uint32_t longest) {
     return tiles < most ? tiles : most;
 }
 
-// Split-KV plan of the attention launch for a round of n_tok tokens (flash-decoding): every CTA walks
-// `tps` 64-position tiles, the grid is deep enough for `max_tiles`, and a token with a shorter context
-// simply uses fewer of its CTAs.  Planned for the round's own contexts, not for the longest that the cache allows, which cut 16
-// sequences of 100 to 290 tokens by four tiles and sent one sequence of 129 through scratch instead of a cluster (8B shape, per
-// round: 3.88 -> 3.71 ms in Q8_0, 2.81 -> 2.73 ms in f16; one sequence of 200 tokens of the 1B shape 657 -> 623 us).
-// Rounds with enough tokens to fill the GPU on their own (prefill) are not split.
 // Fewest tokens in a round for which the linear layers run as batched tensor-core kernels instead of
 // the register-blocked GEMV (measured on the 8B shapes: the GEMV wins up to 2 tokens).
 static int batched_min_tokens() { return 3; }
 
-static void attn_plan(const lcu_ctx *c, int n_tok, int max_tiles, int *n_splits, int *tps) {
-    const int ctas = c->nkvh_l * n_tok;
-    if (ctas >= 8 * sm_count() || max_tiles <= 1) {
-        *n_splits = 1;
-        *tps = max_tiles;
-        return;
-    }
-    // tiles per CTA: enough CTAs to fill the GPU about eight times over when every context is full, at most 4 (four times: 16
-    // sequences of 100 to 290 tokens of the 8B shape 3.76 instead of 3.71 ms per round)
-    int t = (int)(((long)ctas * max_tiles + 8L * sm_count() - 1) / (8L * sm_count()));
-    if (t > 4) t = 4;
-    if (t < 1) t = 1;
-    // a round of a few tokens merges its splits inside one thread-block cluster (at most 8 CTAs): take 2 tiles per
-    // CTA when that is what it needs
-    if (n_tok < batched_min_tokens() && t == 1 && max_tiles > 8 && max_tiles <= 16) t = 2;
-    int z = (max_tiles + t - 1) / t;
-    int z_cap = 2048 / n_tok;  // bounds the partial-output scratch
-    if (z_cap > 64) z_cap = 64;
-    if (z_cap < 1) z_cap = 1;
-    if (z > z_cap) {
-        z = z_cap;
-        t = (max_tiles + z - 1) / z;
-    }
-    *n_splits = z;
-    *tps = t;
+static AttnPlan attn_plan_of(const lcu_ctx *c, int n_tok, int max_tiles) {
+    return attn_plan(c->nkvh_l, c->desc.dh, n_tok, max_tiles, sm_count(), !(c->batched_ok && n_tok >= batched_min_tokens()));
 }
 
 static int attn_splits(const lcu_ctx *c, int n_tok) {  // the deepest of every length of contexts
     int most = 1;
     const int tiles = attn_tiles(c, (uint32_t)c->desc.nctx);
     for (int m = 1; ; m = m * 2 < tiles ? m * 2 : tiles) {
-        int z, t;
-        attn_plan(c, n_tok, m < tiles ? m : tiles, &z, &t);
+        const int z = attn_plan_of(c, n_tok, m < tiles ? m : tiles).splits;
         if (z > most) most = z;
         if (m >= tiles) return most;
     }
@@ -725,8 +695,7 @@ int enqueue_round(lcu_ctx *c, const Round &r, lcu_kv_pair *out_dev, cudaStream_t
         return reinterpret_cast<unsigned char *>(base) + (size_t)t * stride_elems * eb;
     };
 
-    int n_splits, attn_tps;
-    attn_plan(c, r.n_tok, r.attn_tiles, &n_splits, &attn_tps);
+    const int n_splits = r.attn.splits, attn_tps = r.attn.tiles;
     const bool batched = c->batched_ok && r.n_tok >= batched_min_tokens();
     // GEMV rounds: the three GEMV -> GEMV edges (the edges around attention lose there); batched rounds: also attention -> O
     const int pdl_edges = pdl_edges_env >= 0 ? pdl_edges_env : (batched ? 30 : 28);
@@ -1115,7 +1084,7 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
     Round r;
     r.n_tok = n_tok; r.n_req = n_req; r.n_fast = n_fast; r.any_sampling = any_sampling; r.decode_only = decode_only;
     r.n_groups = 0;
-    r.attn_tiles = attn_tiles(c, longest);
+    if (!c->stack) r.attn = attn_plan_of(c, n_tok, attn_tiles(c, longest));
     r.n_out = rows ? n_rows : n_req;
     r.logits_f32 = logits_dev;
     r.L = desc_layout(n_tok, n_req, r.n_out, c->pt_stride);
@@ -1147,8 +1116,13 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
             if (rc) return rc;
         }
         // prompts in the round: consecutive tokens of a request are grouped for the prefill form of attention
-        r.attn_tc = !c->stack && !decode_only && attn_tc_takes(c->geom, c->n_pages, c->pool, longest);
-        if (!c->stack && !decode_only && (r.attn_tc || attn_prefill_supported(c->pt_stride))) {
+        AttnForm form = ATTN_SPLIT;
+        if (!c->stack && !decode_only) {
+            const bool rows64 = attn_prefill_supported(c->pt_stride), rows256 = attn_tc_takes(c->geom, c->n_pages, c->pool);
+            form = rows256 && tuning().attn_tc == 2 ? ATTN_ROWS256 : attn_form(d.dh, c->nh_l / c->nkvh_l, c->nkvh_l, reqs, n_req, sm_count(), rows64, rows256);
+        }
+        r.attn_tc = form == ATTN_ROWS256;
+        if (form != ATTN_SPLIT) {
             int32_t *hg = reinterpret_cast<int32_t *>(H + r.L.groups);
             const int gt = r.attn_tc ? attn_tc_group_tokens(c->nh_l, c->nkvh_l) : attn_prefill_group_tokens(c->nh_l, c->nkvh_l);
             int t0 = 0;
@@ -1209,7 +1183,8 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
         return finish(rc);
     }
     std::vector<int> key = {n_req, n_tok, n_fast, any_sampling ? 1 : 0, (int)((uintptr_t)out_dev & 0x7fffffff),
-                            (int)((uintptr_t)out_dev >> 31), c->head_shard ? 1 : 0, c->stack ? 0 : r.attn_tiles};
+                            (int)((uintptr_t)out_dev >> 31), c->head_shard ? 1 : 0, c->stack ? 0 : r.attn.splits,
+                            c->stack || r.attn.splits == 1 ? 0 : r.attn.tiles};  // (one split walks the whole context, whatever its length)
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
         // A captured round is keyed by its shape, the reach of its attention AND by the output buffer (a host that rotates output buffers, as the

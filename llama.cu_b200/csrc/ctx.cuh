@@ -101,7 +101,7 @@ struct Round {
     int n_tok, n_req, n_fast;
     int n_out;     // rows of logits: one per request, or what lcu_step_logits asks for
     int n_groups;  // token groups for the prefill form of attention (0: decode form)
-    int attn_tiles;  // tiles of 64 positions that the decode form's splits reach
+    AttnPlan attn{1, 1};  // how the decode form cuts contexts
     bool attn_tc = false;  // ... on tcgen05 (attention_tc.cu)
     bool any_sampling;
     bool decode_only;  // one new token per sequence
