@@ -134,11 +134,7 @@ static bool is_linear_kind(int kind) {
 }
 
 // captured graphs hold weight pointers: any change of registered memory drops them
-static void drop_graphs(lcu_ctx *c) {
-    for (auto &g : c->graphs)
-        if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
-    c->graphs.clear();
-}
+static void drop_graphs(lcu_ctx *c) { c->graphs.clear(); }
 
 static void p2p_release(lcu_ctx *c) {
     P2pState &st = c->p2p;
@@ -372,8 +368,7 @@ int lcu_ctx_destroy(lcu_ctx *c) {
     if (!c) return LCU_OK;
     cudaSetDevice(c->device);
     cudaDeviceSynchronize();
-    for (auto &g : c->graphs)
-        if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
+    drop_graphs(c);
     for (int i = 0; i < lcu_ctx::RING; ++i) {
         if (c->desc_host[i]) cudaFreeHost(c->desc_host[i]);
         if (c->desc_event[i]) cudaEventDestroy(c->desc_event[i]);
@@ -1185,11 +1180,10 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
     std::vector<int> key = {n_req, n_tok, n_fast, any_sampling ? 1 : 0, (int)((uintptr_t)out_dev & 0x7fffffff),
                             (int)((uintptr_t)out_dev >> 31), c->head_shard ? 1 : 0, c->stack ? 0 : r.attn.splits,
                             c->stack || r.attn.splits == 1 ? 0 : r.attn.tiles};  // (one split walks the whole context, whatever its length)
-    auto it = c->graphs.find(key);
-    if (it == c->graphs.end()) {
-        // A captured round is keyed by its shape, the reach of its attention AND by the output buffer (a host that rotates output buffers, as the
-        // reference's triple-buffered loop does, holds one graph per buffer): keep the table bounded
-        if (c->graphs.size() >= 96) drop_graphs(c);
+    StepGraph *round = c->graphs.find(key);
+    if (!round) {
+        // A captured round is keyed by its shape, the split of its attention AND by the output buffer (a host that rotates output buffers,
+        // as the reference's triple-buffered loop does, holds one graph per buffer); the table is bounded
         cudaGraph_t graph = nullptr;
         LCU_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         int count = 0;
@@ -1205,10 +1199,10 @@ static int run_step(lcu_ctx *c, lcu_stream_t stream, int n_req, const lcu_req *r
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
         g.launches = count;
-        it = c->graphs.emplace(key, g).first;
+        round = c->graphs.insert(key, g);
     }
-    LCU_CHECK_CUDA(cudaGraphLaunch(it->second.exec, s));
-    c->last_launches = it->second.launches;
+    LCU_CHECK_CUDA(cudaGraphLaunch(round->exec, s));
+    c->last_launches = round->launches;
     return finish(LCU_OK);
 }
 

@@ -7,6 +7,7 @@
 #include "attention.cuh"
 #include "common.cuh"
 #include "p2p.cuh"
+#include "round_table.hpp"
 #include "stack.cuh"
 
 struct LayerWeights {
@@ -27,6 +28,13 @@ struct SeqState {
 struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     int launches = 0;
+};
+
+struct DropGraph {
+    void operator()(StepGraph &g) const {  // (one in flight is freed when it has ended)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
 };
 
 struct lcu_ctx {
@@ -84,7 +92,9 @@ struct lcu_ctx {
     std::vector<int> free_slots;      // recurrent-state slots
 
     bool use_graph = true;
-    std::map<std::vector<int>, StepGraph> graphs;
+    // captured rounds: three output buffers, 33 batch sizes and the two attention splits that a service moves between (a round of 32
+    // layers: 1.5 to 3 ms to capture, 0.14 MB of device and 2 MB of host memory)
+    lcu::RoundTable<StepGraph, DropGraph> graphs{200, DropGraph()};
     int last_launches = 0;
     double last_bytes = 0;
     int last_n_tok = 0, last_n_req = 0;
