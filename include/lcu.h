@@ -328,7 +328,7 @@ LCU_API int lcu_set_wait_limit_us(lcu_ctx *ctx, long long us);
 /* Process-wide tuning values; the defaults are what the committed measurements use.  Keys: "pdl_edges" (bit per
  * layer edge launched as a programmatic dependent: 0 QKV->attention, 1 attention->O, 2 O->gate|up, 3 gate|up->down,
  * 4 down->next QKV, 5 last down->LM head; -1 = default), "gemv_ctas_per_sm" (1, 2; read at a shape's first launch),
- * "q8_rows" (1, 2, 4), "tc" (0: no tcgen05 kernel), "tc_block" (64, 128, 256), "tc_pair_min" (fewest tokens of a launch that takes pairs of SMs, 0: none), "tc_cluster" (0..2), "attn_tc" (0..2: tcgen05 attention of prompts never, where faster, always),
+ * "q8_rows" (1, 2, 4), "tc" (0: no tcgen05 kernel), "tc_block" (64, 128, 256), "tc_pair_min" (fewest tokens of a launch that takes pairs of SMs, 0: none; 1: every launch, however few its tiles), "tc_cluster" (0..2), "attn_tc" (0..2: tcgen05 attention of prompts never, where faster, always),
  * "p2p_scatter_ranks", "p2p_scatter_min", "gemv_lean_norm" (0: general RMSNorm prologue in the one-token GEMV),
  * "rms_pdl" (0: the stand-alone RMSNorm of batched rounds is a plain launch), "expand_min" (latent attention: fewest tokens of
  * a portion that expands keys and values; 0 = from the operation counts, -1 = never), "latent_tc" (0: mma.sync kernel in decode

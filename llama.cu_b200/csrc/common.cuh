@@ -165,6 +165,9 @@ __device__ __forceinline__ uint32_t ld_stream_32(const void *p) {
 // attribute may start while its predecessor drains; everything it does before
 // grid_dep_wait() must touch only memory no earlier kernel of the step writes (weights).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel that owns tensor memory may call this before it allocates only because no dependent that allocates fits on the same SM: all
+// of them take more than half of its shared memory (gemm_tc.cu, gemm_pair.cu, attention_tc.cu, latent_tc.cu: 147 KB and more).  One
+// that fitted could hold the columns that this kernel's next block waits for, and wait for this kernel.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float warp_sum(float v) {

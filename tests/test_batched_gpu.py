@@ -79,11 +79,16 @@ def test_8b_cut_12_and_40_sequences(L, O, n):
     run_case(L, O, cfg, ragged_lengths(n, [270, 70], seed=n), 8, True)
 
 
-def test_8b_q8_cut_16_sequences(L, O):
-    """Q8_0 weights, 16 sequences: the mma.sync kernel's Q8_0 form in every projection."""
+@pytest.mark.parametrize("tc", [1, 0])
+def test_8b_q8_cut_16_sequences(L, O, tc):
+    """Q8_0 weights, 16 sequences: the tcgen05 kernel in every projection, or the mma.sync kernel's Q8_0 form."""
     from llama_cu_b200.model import reduced
     cfg = reduced(L.CONFIGS["llama8b_q8"], 2, 4096)
-    run_case(L, O, cfg, ragged_lengths(16, [300, 130]), 8, True)
+    L.set_tuning("tc", tc)
+    try:
+        run_case(L, O, cfg, ragged_lengths(16, [300, 130]), 8, True)
+    finally:
+        L.set_tuning("tc", 1)
 
 
 def test_1b_cut_bf16_24_sequences(L, O):

@@ -1,5 +1,6 @@
-"""Linear layers of 9 to 128 tokens on tcgen05: every split of K over a cluster (1 to 8 CTAs), whole and cut row blocks, and the
-stream-K form beside it, against f64 products."""
+"""Linear layers of 9 to 128 tokens on tcgen05 as the stand-alone operator runs them, against f64 products: 1 to 300 row blocks, which the
+cost rule gives to clusters of 1 to 8 CTAs or to whole row blocks.  The operator has no scratch, so row blocks are never cut here:
+those are in test_linear_round_gpu.py."""
 import ctypes as C
 
 import pytest
