@@ -52,7 +52,7 @@ struct AttnCost {
 template <class Req>  // with `pos` cached tokens and `len` new ones
 double attn_form_cost(AttnForm form, int dh, int group, int nkvh, const Req *reqs, int n_req, int sms) {
     static const AttnCost rows64[2] = {{2.3, 0.7, 0.7, 0.4, 1.65}, {1.8, 1.4, 1.4, 0.0, 1.85}};
-    static const AttnCost rows256[2] = {{5.9, 0.8, 2.0, 2.9, 1.2}, {4.2, 1.5, 2.5, 1.2, 1.35}};
+    static const AttnCost rows256[2] = {{5.9, 0.8, 2.0, 2.9, 1.2}, {4.2, 1.5, 2.5, 0.8, 1.55}};
     const bool big = form == ATTN_ROWS256;
     const AttnCost &c = (big ? rows256 : rows64)[dh == 64 ? 0 : 1];
     const long per = (big ? 256 : 64) / group, tile = big ? 128 : 64;

@@ -91,7 +91,7 @@ def test_form_follows_rows_and_contexts(ask, dh, group, nkvh, reqs, want):
 
 
 @pytest.mark.parametrize("nkvh,reqs,want", [
-    (8, [(60000, 4), (5, 1)], SPLIT), (8, [(60000, 16)], SPLIT), (8, [(20000, 8)], SPLIT), (8, [(60000, 1)] * 6 + [(0, 20)], SPLIT), (32, [(60000, 2)], SPLIT),
+    (8, [(60000, 4), (5, 1)], SPLIT), (8, [(60000, 16)], SPLIT), (8, [(20000, 8)], SPLIT), (8, [(20000, 16)], SPLIT), (8, [(60000, 1)] * 6 + [(0, 20)], SPLIT), (32, [(60000, 2)], SPLIT),
     (8, [(60000, 64)], ROWS256), (8, [(5000, 128)], ROWS256), (32, [(60000, 16)], ROWS256), (8, [(0, 60000)], ROWS256)])
 def test_few_tokens_behind_a_long_context_are_split(ask, nkvh, reqs, want):
     """More pages than the 64-row form takes: without the decode form, four tokens behind 60000 take 1.67 instead of 0.48 ms."""
